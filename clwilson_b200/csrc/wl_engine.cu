@@ -115,21 +115,41 @@ int ensure_columns(wl_ctx* c, uint64_t limit) {
     c->sieve_bytes += 2ull * nseg * SEG_WORDS * 4 + 2ull * nseg * 4 + 2ull * (nseg + 1) * 8 + total * 4;
     c->ncols = total;
     c->col_limit = nl;
-    // the exact products of the table's aligned column groups
     c->ngroups = 0;
-    const uint64_t ng = total / COL_GROUP;
-    RC(ensure(c->gprod, (size_t)ng * COL_GROUP * 4 + 16));
-    RC(ensure(c->gk, (size_t)ng + 16));
-    launch_group_products(as<uint32_t>(c->cols), ng, as<uint32_t>(c->gprod), as<uint8_t>(c->gk), c->st);
-    c->launches++;
-    c->ngroups = ng;
     return 0;
+}
+
+ColGroups col_groups(wl_ctx* c) {
+    static const bool off = getenv("WL_COL_GROUPS") && atoi(getenv("WL_COL_GROUPS")) == 0;
+    ColGroups g;
+    if (off) return g;
+    const uint64_t ng = c->ncols / COL_GROUP;
+    if (c->ngroups != ng) {
+        if (ensure(c->gprod, (size_t)ng * COL_GROUP * 4 + 16) || ensure(c->gk, (size_t)ng + 16)) return g;
+        launch_group_products(as<uint32_t>(c->cols), ng, as<uint32_t>(c->gprod), as<uint8_t>(c->gk), c->st);
+        c->launches++;
+        c->ngroups = ng;
+    }
+    if (!ng) return g;
+    g.gprod = as<uint32_t>(c->gprod);
+    g.gk = as<uint8_t>(c->gk);
+    g.ngroups = ng;
+    return g;
 }
 
 // ---------------------------------------------------------------------------
 // the search pipeline over a set of ranges
 // ---------------------------------------------------------------------------
 
+
+// The tensor-core product's launches and the wait for its counts take about
+// 0.25 ms of a call: it runs where it saves more (WL_TENSOR=0 in the environment
+// turns it off, for comparisons).
+constexpr double TENSOR_MIN_SAVING_MS = 0.3;
+static bool tensor_enabled() {
+    static const bool off = getenv("WL_TENSOR") && atoi(getenv("WL_TENSOR")) == 0;
+    return !off;
+}
 
 struct HostBucket {
     uint32_t range, type, L;
@@ -563,6 +583,26 @@ static int run_ranges(wl_ctx* c, const wl_range* ranges, size_t nr, uint64_t qca
     }
 
     // ---- 4. device layout: rows, buckets, splits, items ------------------------
+    // buckets with enough work take the tensor-core product (wl_tensor.cu) and
+    // leave the sweeps without columns
+    size_t free_b = 0, total_b = 0;
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) { cudaGetLastError(); free_b = 8ull << 30; }
+    std::vector<TensorTask> tensor;
+    std::vector<char> on_tensor(nb, 0);
+    const size_t tbudget = tensor_budget(c, free_b);
+    if (tbudget && tensor_enabled()) {
+        double saved = 0;
+        for (size_t i = 0; i < nb; ++i) {
+            const double ms = tensor_saves((uint32_t)hb[i].primes.size(), (int)hb[i].L, hb[i].T, cb_lo[i],
+                                           ncol[i] - ndn[i], ndn[i]);
+            on_tensor[i] = ms > 0;
+            if (ms > 0) saved += ms;
+        }
+        if (saved < TENSOR_MIN_SAVING_MS) std::fill(on_tensor.begin(), on_tensor.end(), 0);
+    }
+    std::vector<uint64_t> all_cols(ncol.begin(), ncol.begin() + nb);   // what each bucket multiplies in all
+    for (size_t i = 0; i < nb; ++i)
+        if (on_tensor[i]) ncol[i] = ndn[i] = 0;
     std::vector<Bucket> db(hb.size());
     std::vector<RowInfo> ri(nrows);
     std::vector<uint64_t> row_src(nrows);    // global output index (range-major, ascending p)
@@ -615,8 +655,6 @@ static int run_ranges(wl_ctx* c, const wl_range* ranges, size_t nr, uint64_t qca
     }
     double scale = 1.0;
     {
-        size_t free_b = 0, total_b = 0;
-        if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) { cudaGetLastError(); free_b = 8ull << 30; }
         const double budget = std::min<double>((double)(free_b + c->part.cap) / 3.0, 24.0 * (1ull << 30)) / 16.0;
         scale = split_scale(sbs, W, target_threads, budget);
     }
@@ -637,7 +675,7 @@ static int run_ranges(wl_ctx* c, const wl_range* ranges, size_t nr, uint64_t qca
         const int rpt = sparse_rpt_for(c->tune.sparse_rpt[b.L - 2], b.nrows);
         const uint64_t nd = ndn[i];
         uint64_t Sd = 0, Ss = 0;
-        plan_splits(i, scale, &Sd, &Ss);
+        if (!on_tensor[i]) plan_splits(i, scale, &Sd, &Ss);
         b.cdense = (uint32_t)nd;
         b.ndense = (uint32_t)Sd;
         b.dstart = (uint32_t)dkeys_bucket_start.size();
@@ -657,7 +695,18 @@ static int run_ranges(wl_ctx* c, const wl_range* ranges, size_t nr, uint64_t qca
         b.def_base = def_total;
         part_total += S * b.nrows;
         def_total += (uint32_t)S;
-        out.cells += (uint64_t)b.nrows * b.ncols;
+        out.cells += (uint64_t)b.nrows * all_cols[i];
+        if (on_tensor[i]) {
+            TensorTask t;
+            t.T = b.T;
+            t.c0 = cb_lo[i];
+            t.c1 = cb_lo[i] + all_cols[i];
+            t.row_begin = b.row_begin;
+            t.nrows = b.nrows;
+            t.L = (int)b.L;
+            t.q_max = (uint32_t)std::min<uint64_t>(keys[i], 0xFFFFFFFFull);
+            tensor.push_back(t);
+        }
         std::vector<RowTile> tiles;
         if (Ss) {
             const double per_split = (double)(b.ncols - b.cdense) / (double)Ss;   // sparse: equal splits
@@ -792,12 +841,22 @@ static int run_ranges(wl_ctx* c, const wl_range* ranges, size_t nr, uint64_t qca
     // per-row accumulators of the column products (1, or the resumed products)
     RC(ensure(c->uacc, (size_t)nrows * 16 + 16));
     RC(ensure(c->udef, db.size() * sizeof(Deficit) + 16));
-    RC(ensure(c->work, 24));
+    RC(ensure(c->work, 32));
+    CK(cudaMemsetAsync(c->work.p, 0, 32, c->st));
+    // the groups' exact products take 16 multiplies a column and save a tenth of
+    // the cells; they stay with the table for later calls
+    ColGroups col_grp;
+    {
+        double sparse = 0;
+        for (const SplitBucket& b : sbs) sparse += (double)b.nrows * (double)b.nsparse;
+        if (sparse >= 8.0 * (double)c->ncols) col_grp = col_groups(c);
+    }
     // from here to the lift the device work is fixed by the plan above: a
     // batch issues it as one graph (no initial products to upload and no
     // columns above 2^32, whose windows are planned from device counts)
     ChainGraph cg;
-    if (graph && !init && !big_need) RC(cg.begin(c->st));
+    const bool as_graph = graph && !init && !big_need;
+    if (as_graph && tensor.empty()) RC(cg.begin(c->st));
     launch_acc_init(nrows, (uint32_t)db.size(), as<uint4>(c->uacc), as<Deficit>(c->udef), c->st);
     c->launches++;
     if (init) {
@@ -814,9 +873,13 @@ static int run_ranges(wl_ctx* c, const wl_range* ranges, size_t nr, uint64_t qca
     }
     launch_setup_rows(as<RowInfo>(c->rowinfo), nrows, as<RowMod>(c->rowmod), c->st);
     c->launches++;
-    CK(cudaMemsetAsync(c->work.p, 0, 24, c->st));
     CK(cudaEventRecord(c->rows_ready, c->st));
     cg.record(c->ev[2], c->st);
+    if (!tensor.empty()) {
+        // planned from counts that the device makes, so outside the graph
+        RC(tensor_products(c, tensor, nrows, tbudget));
+        if (as_graph) RC(cg.begin(c->st));
+    }
     size_t ioff = 0;
     bool forked = false;
     for (auto& g : groups) {
@@ -833,7 +896,7 @@ static int run_ranges(wl_ctx* c, const wl_range* ranges, size_t nr, uint64_t qca
         else
             launch_sweep(c->tune.sparse_variant[g.L - 2], g.L, g.rpt, (uint32_t)g.items.size(), as<Bucket>(c->buckets),
                          as<SweepItem>(c->items) + ioff, as<RowMod>(c->rowmod), as<uint32_t>(c->cols),
-                         as<uint4>(c->part), as<Deficit>(c->defs), c->st, col_groups(c));
+                         as<uint4>(c->part), as<Deficit>(c->defs), c->st, col_grp);
         if (!g.items.empty()) c->launches++;
         ioff += g.items.size();
     }
@@ -903,12 +966,14 @@ static int run_ranges(wl_ctx* c, const wl_range* ranges, size_t nr, uint64_t qca
     std::vector<RowOut> ro(nrows);
     CK(cudaMemcpyAsync(ro.data(), c->rowout.p, (size_t)nrows * sizeof(RowOut), cudaMemcpyDeviceToHost, c->st));
     c->d2h += (size_t)nrows * sizeof(RowOut);
-    unsigned long long dwork[3] = { 0, 0, 0 };
-    CK(cudaMemcpyAsync(dwork, c->work.p, 24, cudaMemcpyDeviceToHost, c->st));
-    c->d2h += 24;
+    unsigned long long dwork[4] = { 0, 0, 0, 0 };
+    CK(cudaMemcpyAsync(dwork, c->work.p, 32, cudaMemcpyDeviceToHost, c->st));
+    c->d2h += 32;
     cudaEventRecord(c->ev[5], c->st);
     CK(cudaStreamSynchronize(c->st));
     CK(cudaGetLastError());
+
+    if (dwork[3]) return WL_ERR_CUDA;   // a wait of the tensor-core product ran out
 
     // ---- 6. gather rows in range order, ascending p ------------------------------
     out.rows.assign(nrows, wl_row{});
@@ -1101,7 +1166,9 @@ void wl_close(wl_ctx* c) {
                        &c->buckets, &c->rowinfo, &c->rowmod, &c->items, &c->part, &c->ipart, &c->dsplit,
                        &c->bbitmap, &c->bsegcount, &c->boffsets, &c->boffs, &c->wcols, &c->wbuckets, &c->witems,
                        &c->wpart, &c->wdefs, &c->bacc, &c->bdef, &c->wkeys, &c->wcounts, &c->uacc, &c->udef,
-                       &c->defs, &c->rowout, &c->prod, &c->windesc, &c->seglo, &c->work };
+                       &c->defs, &c->rowout, &c->prod, &c->windesc, &c->seglo, &c->work,
+                       &c->tb.desc, &c->tb.counts, &c->tb.tables, &c->tb.list, &c->tb.w, &c->tb.consts, &c->tb.ones,
+                       &c->tb.part, &c->tb.seg, &c->tb.win, &c->gprod, &c->gk };
     for (DevBuf* b : bufs) if (b->p) cudaFree(b->p);
     for (auto& e : c->ev) if (e) cudaEventDestroy(e);
     if (c->fork) cudaEventDestroy(c->fork);

@@ -10,6 +10,7 @@
 
 #include "wilson.h"
 #include "wl_internal.h"
+#include "wl_tensor.h"
 
 // A growable device buffer.
 struct DevBuf {
@@ -116,6 +117,11 @@ inline int limb_width(uint64_t pmax_incl) {
         if (r_) return r_;         \
     } while (0)
 
+// Workspace of the tensor-core column products (wl_tensor_host.cu).
+struct TensorBufs {
+    DevBuf desc, counts, tables, list, w, consts, ones, part, seg, win;
+};
+
 struct wl_ctx {
     int device = 0;
     int sms = 148;
@@ -133,7 +139,7 @@ struct wl_ctx {
     DevBuf cols;            // column cache: all primes < col_limit, ascending, u32
     uint64_t ncols = 0, col_limit = 0;
     DevBuf gprod, gk;       // exact products of its aligned groups of COL_GROUP columns
-    uint64_t ngroups = 0;
+    uint64_t ngroups = 0;   // 0 until a prefix-fold sweep asks for them (col_groups)
     DevBuf bitmap, segcount, offsets;
     DevBuf tp, keys, counts, buckets, rowinfo, rowmod, items, part, ipart, defs, rowout, dsplit;
     // columns above 2^32
@@ -146,20 +152,18 @@ struct wl_ctx {
     uint64_t h2d = 0, d2h = 0;
     double ms_sieve = 0;
     uint64_t sieve_ints = 0, sieve_bytes = 0;
-    DevBuf work;         // dense sweep work counters: column cells, window cells, products
+    DevBuf work;         // dense sweep work counters: column cells, window cells, products; then the
+                         // tensor-core product's error word
+    TensorBufs tb;
 };
 
-// The column groups of the resident table for the prefix-fold sweep
-// (WL_COL_GROUPS=0 in the environment turns them off, for comparisons).
-inline wl::ColGroups col_groups(wl_ctx* c) {
-    static const bool off = getenv("WL_COL_GROUPS") && atoi(getenv("WL_COL_GROUPS")) == 0;
-    wl::ColGroups g;
-    if (off || !c->ngroups) return g;
-    g.gprod = as<uint32_t>(c->gprod);
-    g.gk = as<uint8_t>(c->gk);
-    g.ngroups = c->ngroups;
-    return g;
-}
+// Every prime below `limit` (<= 2^32) in the context's resident column table.
+int ensure_columns(wl_ctx* c, uint64_t limit);
+// The column groups of the resident table for the prefix-fold sweep, built on
+// the main stream when first asked for after the table was; none (every column
+// one cell) when there is no memory for them or with WL_COL_GROUPS=0 in the
+// environment, for comparisons.
+wl::ColGroups col_groups(wl_ctx* c);
 
 // A range's window of test primes and its classes.
 struct RangeState {
@@ -171,11 +175,19 @@ struct RangeState {
     uint64_t per_class[3] = { 0, 0, 0 };
 };
 
-// Every prime below `limit` (<= 2^32) in the context's resident column table.
-int ensure_columns(wl_ctx* c, uint64_t limit);
 // Test primes of each range, ascending (deterministic Miller-Rabin on the
 // device); with allow_empty a range without primes is not an error.
 int gen_test_primes(wl_ctx* c, const wl_range* ranges, size_t nr, std::vector<RangeState>& rs,
                     std::vector<uint64_t>& tps, bool allow_empty = false);
+// Workspace the tensor-core products may take with `free_bytes` of device
+// memory free; 0: too little, the sweeps run instead.
+size_t tensor_budget(wl_ctx* c, size_t free_bytes);
+// Modelled time that the tensor-core product saves over the sweeps for a bucket
+// of nrows rows over nsparse + ndense columns from index c0 on, in ms (negative:
+// the sweeps are faster).
+double tensor_saves(uint32_t nrows, int L, uint64_t T, uint64_t c0, uint64_t nsparse, uint64_t ndense);
+// Multiplies each task's columns into its rows' accumulators (uacc), on the
+// main stream; rowmod must be set up.  Row indices are below nrows_total.
+int tensor_products(wl_ctx* c, std::vector<wl::TensorTask> tasks, uint32_t nrows_total, size_t budget);
 // results.txt value of one row (cl_wilson.cpp:872-898): 1 if it is a result line.
 int result_of(const wl_row& r, int32_t* value);

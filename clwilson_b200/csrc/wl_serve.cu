@@ -309,6 +309,9 @@ static void serve_admit_batch(wl_server* s, const std::vector<SReq*>& cands, std
         fail_admitted(WL_ERR_CUDA);
         return;
     }
+    // the pipeline is drained here: build the column groups now rather than in a step
+    for (size_t i = 0; i < nk; ++i)
+        if (cnt[nk + i] < cnt[i]) { (void)col_groups(c); break; }
     // 4. buckets, rows and tail items on the host (tail items indexed globally
     // in the admission's tail buffer)
     std::vector<std::vector<RowInfo>> ris(adm.size());

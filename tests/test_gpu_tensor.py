@@ -1,0 +1,75 @@
+"""Column products on the tensor cores (wl_tensor.cu), bit for bit against the oracle.
+
+Ranges large enough that every class takes that path, which the call's stats
+show (no dense sweep ran although every capped column here is in its regime),
+at the edges of the limb widths (p just below 2^31, 2^47 and 2^62), with few
+and many rows per 256-column tile, with 5- to 9-bit exponent digits, with
+columns cut off at odd places and starting past 2 with a running product.
+"""
+import numpy as np
+import pytest
+
+import oracle
+
+pytestmark = pytest.mark.gpu
+TOP = (1 << 62) - 1
+
+
+@pytest.fixture(scope="module", autouse=True)
+def built():
+    oracle.build()
+
+
+def _same(got, want, sel, fields=("p", "s0", "s1")):
+    for f in fields:
+        assert np.array_equal(got[f][sel].astype(np.uint64), want[f][sel].astype(np.uint64)), f
+
+
+@pytest.mark.parametrize("lo,hi,qcap,nsample", [
+    ((1 << 31) - 800001, (1 << 31) - 1, (1 << 16) + 1, 200),  # 2 limbs, n up to 2^62, short lists
+    ((1 << 47) - 60001, (1 << 47) - 1, (1 << 20) + 7, 6),     # 3 limbs, n up to 2^94
+    (10**13, 10**13 + 800000, 1 << 16, 200),                  # 27,000 rows, 5-bit digits
+    (10**13, 10**13 + 30000, (1 << 22) - 1, 6),
+    (TOP - 8000, TOP, 1 << 24, 6),                            # 46 to 93 rows per class, 9-bit digits
+    (TOP - 60000, TOP, 1 << 20, 6),                           # 4 limbs, n up to 2^124
+], ids=["2^31", "2^47", "mid-16", "mid-22", "top-few-rows", "top"])
+def test_capped_products(engine, lo, hi, qcap, nsample):
+    rows, st = engine.rows(lo, hi, q_cap=qcap)
+    assert st.dense_column_cells == 0
+    sel = (np.linspace(0, len(rows) - 1, nsample).astype(np.uint32) if nsample
+           else np.arange(len(rows), dtype=np.uint32))
+    want, _ = oracle.search(lo, hi, qcap, rows=sel)
+    _same(rows, want, sel)
+
+
+@pytest.mark.parametrize("lo,hi,nsample", [(3 * 10**6, 3 * 10**6 + 60000, 0), (3 * 10**8, 3 * 10**8 + 50000, 12)])
+def test_full_search(engine, lo, hi, nsample):
+    rows, st = engine.rows(lo, hi)
+    assert (rows["status"] == 0).all() and (rows["rem"] == 0).all()
+    sel = np.linspace(0, len(rows) - 1, nsample).astype(np.uint32) if nsample else np.arange(len(rows), dtype=np.uint32)
+    want, _ = oracle.search(lo, hi, rows=sel)
+    _same(rows, want, sel, ("p", "s0", "s1", "rem", "quot"))
+
+
+def test_resumed_products(engine):
+    lo, hi, cuts = TOP - 40000, TOP - 1, (1000, 1 << 19, (1 << 21) + 12345)
+    part = None
+    q = 2
+    for c in cuts:
+        part, _ = engine.rows_from(lo, hi, q, c, init=part)
+        q = c
+    whole, st = engine.rows(lo, hi, q_cap=cuts[-1])
+    assert st.dense_column_cells == 0
+    _same(part, whole, np.arange(len(whole)))
+    sel = np.linspace(0, len(whole) - 1, 4).astype(np.uint32)
+    want, _ = oracle.search(lo, hi, cuts[-1], rows=sel)
+    _same(whole, want, sel)
+
+
+def test_batch_equals_single_ranges(engine):
+    ranges = [(10**9, 10**9 + 30000), (10**12, 10**12 + 9000), (TOP - 20000, TOP), (10**9 + 50, 10**9 + 90)]
+    per, _, st = engine.batch(ranges, q_cap=1 << 21)
+    assert st.graph_nodes > 0
+    for (a, b), r in zip(ranges, per):
+        one = engine.search(a, b, q_cap=1 << 21)
+        assert r["checksum"] == one.checksum and r["tested"] == one.stats.tested
