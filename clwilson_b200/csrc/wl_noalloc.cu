@@ -1,7 +1,7 @@
 // wl_noalloc.cu -- the column product of one class without any device allocation.
 //
 // wl_column_product_noalloc() runs the same kernels as the engine's capped
-// sweep (k_setup_rows, k_sweep, k_finish) for caller-owned input and output
+// sweep (k_setup_rows, k_sweep_dense, k_sweep, k_finish) for caller-owned input and output
 // buffers, with every intermediate (row constants, split partial products,
 // split deficits, launch descriptors) in one fixed, file-scope device array.
 // It is for callers that cannot allocate device memory while they run: hosts
@@ -16,7 +16,9 @@
 // The input contract is checked on the device, since the inputs live there:
 // a row whose prime is even, below 5 or not below p_bound, and every row when
 // the columns are not ascending primes in [2, T], get s0 = s1 = UINT64_MAX.
+#include <algorithm>
 #include <atomic>
+#include <cmath>
 #include <mutex>
 
 #include "wilson.h"
@@ -56,15 +58,33 @@ __global__ void k_noalloc_clear() {
     *reinterpret_cast<uint32_t*>(g_noalloc_scratch + OFF_FLAG) = 0;
 }
 
-// Fill the bucket, the sweep descriptors and the row records from the
-// caller's primes (so that no host-to-device copy is needed either), and
-// check the inputs: each prime odd in [5, p_bound), the columns ascending in
-// [2, T].
+// One sweep's items: `tiles` row tiles of `nsplit` splits from split0 on,
+// 256 / tps splits to an item when the rows fit one narrow tile.
+struct ItemPlan {
+    uint32_t tps, split0, nsplit, nitems;
+};
+
+__device__ wl::SweepItem plan_item(const ItemPlan& p, uint32_t i) {
+    wl::SweepItem it;
+    it.bucket = 0;
+    it.tps = p.tps;
+    if (p.tps == 256) {
+        it.row0 = (i / p.nsplit) * 256;
+        it.split0 = p.split0 + i % p.nsplit;
+    } else {
+        it.row0 = 0;
+        it.split0 = p.split0 + i * (256 / p.tps);
+    }
+    return it;
+}
+
+// Fill the sweep descriptors (the dense sweep's, then the prefix-fold sweep's)
+// and the row records from the caller's primes (so that no host-to-device copy
+// is needed either), and check the inputs: each prime odd in [5, p_bound), the
+// columns ascending in [2, T].
 __global__ void k_noalloc_prep(const uint64_t* __restrict__ primes, uint32_t nrows, uint64_t p_bound, uint64_t T,
-                               const uint32_t* __restrict__ cols, uint32_t ncols, uint32_t nsplit, uint32_t L,
-                               uint32_t tps, uint32_t nitems) {
+                               const uint32_t* __restrict__ cols, uint32_t ncols, ItemPlan dense, ItemPlan sparse) {
     unsigned char* base = g_noalloc_scratch;
-    wl::Bucket* bk = reinterpret_cast<wl::Bucket*>(base + OFF_BUCKET);
     wl::SweepItem* items = reinterpret_cast<wl::SweepItem*>(base + OFF_ITEMS);
     wl::RowInfo* info = reinterpret_cast<wl::RowInfo*>(base + OFF_INFO);
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -75,37 +95,8 @@ __global__ void k_noalloc_prep(const uint64_t* __restrict__ primes, uint32_t nro
         cols_ok &= q >= 2u && (uint64_t)q <= T && (j == 0 || cols[j - 1] < q);
     }
     if (!cols_ok) *reinterpret_cast<uint32_t*>(base + OFF_FLAG) = 1u;
-    if (i == 0) {
-        wl::Bucket b;
-        b.T = T;
-        b.part_base = 0;
-        b.ncols = ncols;
-        b.row_begin = 0;
-        b.nrows = nrows;
-        b.nsplit = nsplit;
-        b.def_base = 0;
-        b.L = L;
-        b.type = 0;
-        b.range = 0;
-        b.cdense = 0;
-        b.ndense = 0;
-        b.dstart = 0;
-        b.cbase = 0;
-        *bk = b;
-    }
-    if (i < nitems) {
-        wl::SweepItem it;
-        it.bucket = 0;
-        it.tps = tps;
-        if (tps == 256) {
-            it.row0 = (i / nsplit) * 256;
-            it.split0 = i % nsplit;
-        } else {
-            it.row0 = 0;
-            it.split0 = i * (256 / tps);
-        }
-        items[i] = it;
-    }
+    if (i < dense.nitems) items[i] = plan_item(dense, i);
+    else if (i < dense.nitems + sparse.nitems) items[i] = plan_item(sparse, i - dense.nitems);
     if (i < nrows) {
         wl::RowInfo r;
         r.p = primes[i];
@@ -116,6 +107,46 @@ __global__ void k_noalloc_prep(const uint64_t* __restrict__ primes, uint32_t nro
         const bool ok = (r.p & 1) && r.p >= 5 && r.p < p_bound;
         r.type = ok ? 0u : BAD_ROW;
         info[i] = r;
+    }
+}
+
+// The bucket, once the columns are checked: columns up to qd take the dense
+// splits (all of them when there is no other split).  With bad columns it has
+// none, so that the sweeps read nothing that breaks their contract.  One warp;
+// the count of columns <= qd by 32-ary search.
+__global__ void k_noalloc_bucket(uint32_t nrows, uint64_t T, const uint32_t* __restrict__ cols, uint32_t ncols,
+                                 uint32_t qd, uint32_t ndense, uint32_t nsparse, uint32_t L) {
+    const uint32_t lane = threadIdx.x;
+    if (*reinterpret_cast<const uint32_t*>(g_noalloc_scratch + OFF_FLAG)) ncols = 0;
+    uint32_t lo = 0, hi = ncols;          // columns [0, lo) are <= qd, [hi, ncols) are not
+    if (nsparse == 0) lo = hi;
+    if (ndense == 0) hi = lo;
+    while (lo < hi) {
+        const uint32_t step = (hi - lo + 31) / 32;
+        const uint64_t at = (uint64_t)lo + (uint64_t)lane * step;
+        const uint32_t n = __popc(__ballot_sync(0xffffffffu, at < hi && cols[at < hi ? at : lo] <= qd));
+        if (n == 0) { hi = lo; break; }   // cols[lo] > qd
+        const uint32_t last = lo + (n - 1) * step;   // <= qd; the next probe is not
+        hi = min(hi, last + step);
+        lo = last + 1;
+    }
+    if (lane == 0) {
+        wl::Bucket b;
+        b.T = T;
+        b.part_base = 0;
+        b.ncols = ncols;
+        b.row_begin = 0;
+        b.nrows = nrows;
+        b.nsplit = ndense + nsparse;
+        b.def_base = 0;
+        b.L = L;
+        b.type = 0;
+        b.range = 0;
+        b.cdense = lo;
+        b.ndense = ndense;
+        b.dstart = 0;
+        b.cbase = 0;
+        *reinterpret_cast<wl::Bucket*>(g_noalloc_scratch + OFF_BUCKET) = b;
     }
 }
 
@@ -192,25 +223,49 @@ extern "C" int wl_column_product_noalloc(const uint64_t* primes, uint32_t nrows,
         nsplit = s > 0 ? (uint32_t)s : 1;
     }
     if ((uint64_t)nsplit * nrows > NA_MAX_PARTIALS) return WL_ERR_TOO_LARGE;
-    uint32_t tps, nitems;
-    if (nrows >= 256) {
-        tps = 256;
-        nitems = ((nrows + 255) / 256) * nsplit;
-    } else {
-        tps = 1;
-        while (tps < nrows) tps <<= 1;
-        const uint32_t per = 256 / tps;
-        nitems = (nsplit + per - 1) / per;
+    // Columns up to qd, where the exponent changes at most columns, take the dense
+    // sweep: an exponentiation at each of them would make the first of equal
+    // prefix-fold splits several times as long as the rest (2,000 rows, T = 1e8,
+    // 1.08e6 columns: 5.65 ms of sweep, most of it one split).  qd lies a factor
+    // of two above the engine's line, since these few splits are the whole launch.
+    // The splits are shared out by cells (about six to a dense column); the count
+    // of columns below qd that this goes by is an estimate, and any share is right.
+    const double Td = (double)T, qx = 2.0 * std::sqrt(Td * std::log(std::sqrt(Td) + 3.0)) + 16.0;
+    const uint32_t qd = qx < 4294967295.0 ? (uint32_t)qx : 0xFFFFFFFFu;
+    const double nd = std::min((double)ncols, 1.2551 * qx / std::log(qx)), ns = (double)ncols - nd;
+    uint32_t sd = 0;
+    if (ncols > 0) {
+        sd = (uint32_t)(nsplit * 6.0 * nd / (6.0 * nd + ns) + 0.5);
+        sd = std::max<uint32_t>(sd, 1);
+        if (ns <= 0) sd = nsplit;
+        else if (sd >= nsplit) sd = nsplit > 1 ? nsplit - 1 : 0;
     }
+    auto plan = [&](uint32_t split0, uint32_t n, uint32_t min_tps) {
+        ItemPlan p = { 256, split0, n, 0 };
+        if (n == 0) return p;
+        if (nrows >= 256) {
+            p.nitems = ((nrows + 255) / 256) * n;
+        } else {
+            p.tps = min_tps;
+            while (p.tps < nrows) p.tps <<= 1;
+            const uint32_t per = 256 / p.tps;
+            p.nitems = (n + per - 1) / per;
+        }
+        return p;
+    };
+    const ItemPlan dense = plan(0, sd, 8), sparse = plan(sd, nsplit - sd, 1);
+    const uint32_t nitems = dense.nitems + sparse.nitems;
     if (nitems > NA_MAX_ITEMS) return WL_ERR_TOO_LARGE;
 
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const uint32_t prep_threads = nitems > nrows ? nitems : nrows;
+    // enough threads for the items and rows, and for the check of the columns to be short
+    const uint32_t prep_threads = std::max(std::max(nitems, nrows), std::min(ncols / 8, (uint32_t)sms * 1024u));
     // each launch's own error is checked right after it
     k_noalloc_clear<<<1, 1, 0, st>>>();
     if (cudaGetLastError() != cudaSuccess) return WL_ERR_CUDA;
-    k_noalloc_prep<<<(prep_threads + 255) / 256, 256, 0, st>>>(primes, nrows, p_bound, T, cols, ncols, nsplit,
-                                                                (uint32_t)L, tps, nitems);
+    k_noalloc_prep<<<(prep_threads + 255) / 256, 256, 0, st>>>(primes, nrows, p_bound, T, cols, ncols, dense, sparse);
+    if (cudaGetLastError() != cudaSuccess) return WL_ERR_CUDA;
+    k_noalloc_bucket<<<1, 32, 0, st>>>(nrows, T, cols, ncols, qd, sd, nsplit - sd, (uint32_t)L);
     if (cudaGetLastError() != cudaSuccess) return WL_ERR_CUDA;
     wl::Bucket* bk = reinterpret_cast<wl::Bucket*>(base + OFF_BUCKET);
     wl::SweepItem* items = reinterpret_cast<wl::SweepItem*>(base + OFF_ITEMS);
@@ -221,7 +276,9 @@ extern "C" int wl_column_product_noalloc(const uint64_t* primes, uint32_t nrows,
     uint4* part = reinterpret_cast<uint4*>(base + OFF_PART);
     wl::launch_setup_rows(info, nrows, mods, st);
     if (cudaGetLastError() != cudaSuccess) return WL_ERR_CUDA;
-    wl::launch_sweep(1, L, 1, nitems, bk, items, mods, cols, part, defs, st);
+    wl::launch_sweep_dense(L, 1, dense.nitems, bk, items, mods, cols, nullptr, part, defs, st, wl::DENSE_SMEM_W3, 8);
+    if (cudaGetLastError() != cudaSuccess) return WL_ERR_CUDA;
+    wl::launch_sweep(1, L, 1, sparse.nitems, bk, items + dense.nitems, mods, cols, part, defs, st);
     if (cudaGetLastError() != cudaSuccess) return WL_ERR_CUDA;
     wl::launch_finish(L, bk, info, mods, part, defs, 1, nullptr, 0, nrows, 0, out, st);
     if (cudaGetLastError() != cudaSuccess) return WL_ERR_CUDA;
