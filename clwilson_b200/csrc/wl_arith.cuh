@@ -428,6 +428,30 @@ __device__ __forceinline__ void dbl_mod(Res<L>& x, const uint32_t* n) {
     if (geq<L>(x, n)) sub_limbs<L>(x, n);
 }
 
+// R mod n (Montgomery one), R = 2^(32L): the largest power of two below n,
+// doubled up to R -- a few doublings where n fills its limbs.
+template <int L>
+__device__ __forceinline__ Res<L> mont_one(const uint32_t* n) {
+    int top = L - 1;
+    while (top > 0 && n[top] == 0) --top;
+    const int bit = 31 - __clz((int)n[top]);
+    Res<L> x;
+#pragma unroll
+    for (int i = 0; i < L; ++i) x.w[i] = i == top ? 1u << bit : 0u;
+    for (int k = 32 * top + bit; k < 32 * L; ++k) dbl_mod<L>(x, n);
+    return x;
+}
+
+// R^2 mod n from one = R mod n: 2^(32L) in Montgomery form, by squaring 2, 8 or 2
+// (32 L = 2^6, 3 * 2^5, 2^7).
+template <int L>
+__device__ __forceinline__ Res<L> mont_r2(const Res<L>& one, const uint32_t* n, uint32_t ninv) {
+    Res<L> x = one;
+    for (int k = 0; k < (L == 3 ? 3 : 1); ++k) dbl_mod<L>(x, n);
+    for (int k = 0; k < (L == 2 ? 6 : L == 3 ? 5 : 7); ++k) x = mont_mul<L>(x, x, n, ninv);
+    return x;
+}
+
 // base^e (Montgomery domain; one = R mod n), left-to-right binary, e < 2^128
 template <int L>
 __device__ __forceinline__ Res<L> mont_pow(const Res<L>& base, u128 e, const Res<L>& one,
@@ -471,10 +495,10 @@ struct Mod64 {
         m = mod;
         minv = 0 - inv64(mod);
         one = (0 - mod) % mod;
-        // r2 = one * 2^64 mod m by 64 doublings
-        uint64_t x = one;
-        for (int i = 0; i < 64; ++i) { x <<= 1; if (x >= m) x -= m; }
-        r2 = x;
+        // r2 = 2^64 in Montgomery form: 2 squared six times
+        uint64_t x = red64(2 * one, m);
+        for (int i = 0; i < 6; ++i) x = mul64(x, x, m, minv);
+        r2 = red64(x, m);
     }
     __device__ __forceinline__ uint64_t to(uint64_t x) const { return mul64(x % m, r2, m, minv); }
     __device__ __forceinline__ uint64_t from(uint64_t x) const { return red64(mul64(x, 1, m, minv), m); }
@@ -486,16 +510,9 @@ struct Mod64 {
     }
 };
 
-// integer square root of a 64-bit value (Newton from an overestimate)
+// integer square root of a value below 2^63: the double's root is off by one at most
 __device__ __forceinline__ uint64_t isqrt64(uint64_t n) {
-    if (n < 2) return n;
-    int bits = 64 - __clzll(n);
-    uint64_t x = 1ULL << ((bits + 1) / 2);     // x >= sqrt(n)
-    while (true) {
-        uint64_t y = (x + n / x) >> 1;
-        if (y >= x) break;
-        x = y;
-    }
+    uint64_t x = (uint64_t)sqrt((double)n);
     while (x * x > n) --x;
     while ((x + 1) * (x + 1) <= n) ++x;
     return x;

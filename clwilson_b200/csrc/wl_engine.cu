@@ -426,8 +426,8 @@ int gen_test_primes(wl_ctx* c, const wl_range* ranges, size_t nr, std::vector<Ra
     CK(cudaMemcpyAsync(c->windesc.p, wd.data(), nr * sizeof(WinDesc), cudaMemcpyHostToDevice, c->st));
     CK(cudaMemsetAsync(c->bitmap.p, 0, words * 4, c->st));
     CK(cudaMemsetAsync(c->segcount.p, 0, segs * 4, c->st));
-    launch_window_primes_multi(as<WinDesc>(c->windesc), (uint32_t)nr, (uint32_t)blocks, as<uint32_t>(c->bitmap),
-                               as<uint32_t>(c->segcount), c->st);
+    launch_window_primes_multi(as<WinDesc>(c->windesc), (uint32_t)nr, (uint32_t)blocks, as<uint32_t>(c->base), c->nbase,
+                               as<uint32_t>(c->bitmap), as<uint32_t>(c->segcount), c->st);
     c->launches++;
     c->h2d += nr * sizeof(WinDesc);
     std::vector<uint32_t> segcnt(segs);
@@ -466,6 +466,33 @@ int gen_test_primes(wl_ctx* c, const wl_range* ranges, size_t nr, std::vector<Ra
     CK(cudaStreamSynchronize(c->st));
     CK(cudaGetLastError());
     c->d2h += total * 8;
+    return 0;
+}
+
+// Columns <= key for each key, from the resident table (which covers them).
+// Keys below 2^16 are counted on the host, among the sieving primes of the
+// column sieve, so that a small search does not wait for the device here.
+static int count_columns(wl_ctx* c, const std::vector<uint64_t>& keys, std::vector<uint64_t>& out) {
+    out.assign(keys.size(), 0);
+    bool host = true;
+    for (uint64_t k : keys) host &= k < 65536;
+    if (host) {
+        for (size_t i = 0; i < keys.size(); ++i)
+            out[i] = std::upper_bound(c->small.begin(), c->small.end(), (uint32_t)keys[i]) - c->small.begin() +
+                     (keys[i] >= 2 ? 1 : 0);      // small holds the odd primes
+        return 0;
+    }
+    RC(ensure(c->keys, keys.size() * 8));
+    RC(ensure(c->counts, keys.size() * 8));
+    CK(cudaMemcpyAsync(c->keys.p, keys.data(), keys.size() * 8, cudaMemcpyHostToDevice, c->st));
+    launch_count_leq(as<uint32_t>(c->cols), c->ncols, as<uint64_t>(c->keys), (uint32_t)keys.size(),
+                     as<uint64_t>(c->counts), c->st);
+    c->launches++;
+    CK(cudaMemcpyAsync(out.data(), c->counts.p, keys.size() * 8, cudaMemcpyDeviceToHost, c->st));
+    CK(cudaStreamSynchronize(c->st));
+    CK(cudaGetLastError());
+    c->h2d += keys.size() * 8;
+    c->d2h += keys.size() * 8;
     return 0;
 }
 
@@ -556,18 +583,8 @@ static int run_ranges(wl_ctx* c, const wl_range* ranges, size_t nr, uint64_t qca
         keys.push_back(std::min<uint64_t>(qd, keys[i]));
     }
     if (q_lo > 2) keys.push_back(q_lo - 1);   // columns already multiplied in (init)
-    RC(ensure(c->keys, keys.size() * 8));
-    RC(ensure(c->counts, keys.size() * 8));
-    CK(cudaMemcpyAsync(c->keys.p, keys.data(), keys.size() * 8, cudaMemcpyHostToDevice, c->st));
-    launch_count_leq(as<uint32_t>(c->cols), c->ncols, as<uint64_t>(c->keys), (uint32_t)keys.size(),
-                     as<uint64_t>(c->counts), c->st);
-    c->launches++;
-    std::vector<uint64_t> ncol(keys.size());
-    CK(cudaMemcpyAsync(ncol.data(), c->counts.p, keys.size() * 8, cudaMemcpyDeviceToHost, c->st));
-    CK(cudaStreamSynchronize(c->st));
-    CK(cudaGetLastError());
-    c->h2d += keys.size() * 8;
-    c->d2h += keys.size() * 8;
+    std::vector<uint64_t> ncol;
+    RC(count_columns(c, keys, ncol));
     out.pi_maxtarget = ncol[nb];
     uint64_t* ndn = ncol.data() + nb + 1;   // dense column counts per bucket
     // a search resumed at q_lo: each bucket's columns start at cb_lo[i] (the
@@ -585,12 +602,16 @@ static int run_ranges(wl_ctx* c, const wl_range* ranges, size_t nr, uint64_t qca
     // ---- 4. device layout: rows, buckets, splits, items ------------------------
     // buckets with enough work take the tensor-core product (wl_tensor.cu) and
     // leave the sweeps without columns
-    size_t free_b = 0, total_b = 0;
-    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) { cudaGetLastError(); free_b = 8ull << 30; }
+    auto free_memory = []() -> size_t {      // asked for only where it matters: the query is slow
+        size_t free_b = 0, total_b = 0;
+        if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) return free_b;
+        cudaGetLastError();
+        return 8ull << 30;
+    };
     std::vector<TensorTask> tensor;
     std::vector<char> on_tensor(nb, 0);
-    const size_t tbudget = tensor_budget(c, free_b);
-    if (tbudget && tensor_enabled()) {
+    size_t tbudget = 0;
+    if (tensor_enabled()) {
         double saved = 0;
         for (size_t i = 0; i < nb; ++i) {
             const double ms = tensor_saves((uint32_t)hb[i].primes.size(), (int)hb[i].L, hb[i].T, cb_lo[i],
@@ -598,7 +619,8 @@ static int run_ranges(wl_ctx* c, const wl_range* ranges, size_t nr, uint64_t qca
             on_tensor[i] = ms > 0;
             if (ms > 0) saved += ms;
         }
-        if (saved < TENSOR_MIN_SAVING_MS) std::fill(on_tensor.begin(), on_tensor.end(), 0);
+        if (saved >= TENSOR_MIN_SAVING_MS) tbudget = tensor_budget(c, free_memory());
+        if (!tbudget) std::fill(on_tensor.begin(), on_tensor.end(), 0);
     }
     std::vector<uint64_t> all_cols(ncol.begin(), ncol.begin() + nb);   // what each bucket multiplies in all
     for (size_t i = 0; i < nb; ++i)
@@ -655,8 +677,14 @@ static int run_ranges(wl_ctx* c, const wl_range* ranges, size_t nr, uint64_t qca
     }
     double scale = 1.0;
     {
-        const double budget = std::min<double>((double)(free_b + c->part.cap) / 3.0, 24.0 * (1ull << 30)) / 16.0;
-        scale = split_scale(sbs, W, target_threads, budget);
+        // 256 MiB of partials always fit: no need to ask for the free memory
+        const double always = (double)(256ull << 20) / 16.0;
+        scale = split_scale(sbs, W, target_threads, always);
+        if (scale < 1.0) {
+            const double budget =
+                std::min<double>((double)(free_memory() + c->part.cap) / 3.0, 24.0 * (1ull << 30)) / 16.0;
+            scale = split_scale(sbs, W, target_threads, budget);
+        }
     }
     auto plan_splits = [&](size_t i, double sc, uint64_t* Sd_out, uint64_t* Ss_out) {
         plan_bucket_splits(sbs[i], W, target_threads, sc, Sd_out, Ss_out);
@@ -750,20 +778,8 @@ static int run_ranges(wl_ctx* c, const wl_range* ranges, size_t nr, uint64_t qca
     // dense split starts: [0, count(cols <= q_1), ..., cdense] per bucket (device order)
     std::vector<uint32_t> dsplit;
     {
-        std::vector<uint64_t> dcounts(dkeys.size());
-        if (!dkeys.empty()) {
-            RC(ensure(c->keys, dkeys.size() * 8));
-            RC(ensure(c->counts, dkeys.size() * 8));
-            CK(cudaMemcpyAsync(c->keys.p, dkeys.data(), dkeys.size() * 8, cudaMemcpyHostToDevice, c->st));
-            launch_count_leq(as<uint32_t>(c->cols), c->ncols, as<uint64_t>(c->keys), (uint32_t)dkeys.size(),
-                             as<uint64_t>(c->counts), c->st);
-            c->launches++;
-            CK(cudaMemcpyAsync(dcounts.data(), c->counts.p, dkeys.size() * 8, cudaMemcpyDeviceToHost, c->st));
-            CK(cudaStreamSynchronize(c->st));
-            CK(cudaGetLastError());
-            c->h2d += dkeys.size() * 8;
-            c->d2h += dkeys.size() * 8;
-        }
+        std::vector<uint64_t> dcounts;
+        RC(count_columns(c, dkeys, dcounts));
         for (uint32_t oi = 0; oi < db.size(); ++oi) {
             Bucket& b = db[oi];
             const uint32_t k0 = dkeys_bucket_start[oi], n = dkeys_n[oi];
@@ -1150,6 +1166,7 @@ int wl_open(int device, wl_ctx** out) {
         for (uint32_t j = i * i; j < 65536; j += 2 * i) comp[j] = 1;
     }
     c->nbase = (uint32_t)base.size();
+    c->small = base;
     if (ensure(c->base, base.size() * 4) ||
         cudaMemcpy(c->base.p, base.data(), base.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess) {
         wl_close(c);

@@ -63,10 +63,7 @@ struct RowTile {
     uint32_t groups = 0;     // splits per CTA; 0: 256 / tps
 };
 inline uint32_t group_width(uint32_t lanes, uint32_t min_tps) {
-    uint32_t t = min_tps;
-    if (lanes <= 32) { while (t < lanes) t <<= 1; }
-    else t = (lanes + 31) / 32 * 32;
-    return t;
+    return lanes <= 32 ? std::max(lanes, min_tps) : (lanes + 31) / 32 * 32;
 }
 inline void row_tiles(uint32_t n, int rpt, uint32_t min_tps, std::vector<RowTile>& out, bool same_groups = false) {
     out.clear();
@@ -136,6 +133,7 @@ struct wl_ctx {
     double ms_big = 0;
     DevBuf base;            // odd primes < 65536 (sieving primes of the column sieve)
     uint32_t nbase = 0;
+    std::vector<uint32_t> small;   // the same on the host
     DevBuf cols;            // column cache: all primes < col_limit, ascending, u32
     uint64_t ncols = 0, col_limit = 0;
     DevBuf gprod, gk;       // exact products of its aligned groups of COL_GROUP columns

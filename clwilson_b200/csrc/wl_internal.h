@@ -133,8 +133,9 @@ struct WinDesc {
     uint64_t word_off, seg_off;
     uint32_t block0, pad;
 };
-void launch_window_primes_multi(const WinDesc* d, uint32_t nr, uint32_t nblocks, uint32_t* bitmap,
-                                uint32_t* seg_count, cudaStream_t st);
+// base: the nbase odd primes below 2^16, ascending
+void launch_window_primes_multi(const WinDesc* d, uint32_t nr, uint32_t nblocks, const uint32_t* base, uint32_t nbase,
+                                uint32_t* bitmap, uint32_t* seg_count, cudaStream_t st);
 void launch_compact_multi(uint32_t nseg, const uint64_t* seg_lo, const uint32_t* bitmap, const uint64_t* offsets,
                           uint64_t* out64, cudaStream_t st);
 void launch_count_leq(const uint32_t* cols, uint64_t ncols, const uint64_t* keys, uint32_t nkeys,

@@ -393,9 +393,7 @@ k_tensor_consts(const TensorDesc* __restrict__ desc, uint32_t ntask, const RowMo
         uint32_t n[L];
 #pragma unroll
         for (int k = 0; k < L; ++k) n[k] = md.n[k];
-        Res<L> one;                                // R mod n
-        set_small<L>(one, 1);
-        for (int k = 0; k < 32 * L; ++k) dbl_mod<L>(one, n);
+        const Res<L> one = mont_one<L>(n);         // R mod n
         if (sg == 0)
             ones[row] = make_uint4(one.w[0], one.w[1], L > 2 ? one.w[2 < L ? 2 : 0] : 0, L > 3 ? one.w[3 < L ? 3 : 0] : 0);
         Res<L> m256 = one;                         // 256 R mod n
