@@ -142,10 +142,14 @@ ColGroups col_groups(wl_ctx* c) {
 // ---------------------------------------------------------------------------
 
 
-// The tensor-core product's launches and the wait for its counts take about
-// 0.25 ms of a call: it runs where it saves more (WL_TENSOR=0 in the environment
-// turns it off, for comparisons).
-constexpr double TENSOR_MIN_SAVING_MS = 0.3;
+// What a call pays besides its buckets' modelled times (ms).  The sweeps of a
+// small call are serial chains -- a split folds its product at every change of
+// the exponent -- that last 0.3 to 2.5 ms however few the rows are; the
+// tensor-core product's eight launches and its wait about 0.1.  Both measured on
+// calls of 15 to 3,600 rows at 1e5 to 2^62 (1e7, 61 rows: 0.92 against 0.27 ms;
+// 2^62, 30 rows, q < 2^20: 2.10 against 0.41).  WL_TENSOR=0 in the environment
+// turns the tensor-core product off, for comparisons.
+constexpr double SWEEP_CALL_MS = 0.4, TENSOR_CALL_MS = 0.1;
 static bool tensor_enabled() {
     static const bool off = getenv("WL_TENSOR") && atoi(getenv("WL_TENSOR")) == 0;
     return !off;
@@ -612,14 +616,18 @@ static int run_ranges(wl_ctx* c, const wl_range* ranges, size_t nr, uint64_t qca
     std::vector<char> on_tensor(nb, 0);
     size_t tbudget = 0;
     if (tensor_enabled()) {
-        double saved = 0;
+        // all buckets on one path, or, where both have work, each on its faster one
+        double all_tensor = TENSOR_CALL_MS, all_sweeps = SWEEP_CALL_MS, mixed = TENSOR_CALL_MS + SWEEP_CALL_MS;
         for (size_t i = 0; i < nb; ++i) {
-            const double ms = tensor_saves((uint32_t)hb[i].primes.size(), (int)hb[i].L, hb[i].T, cb_lo[i],
-                                           ncol[i] - ndn[i], ndn[i]);
-            on_tensor[i] = ms > 0;
-            if (ms > 0) saved += ms;
+            double a, b;
+            tensor_times((uint32_t)hb[i].primes.size(), (int)hb[i].L, hb[i].T, cb_lo[i], ncol[i] - ndn[i], ndn[i], &a, &b);
+            on_tensor[i] = a < b;
+            all_tensor += a;
+            all_sweeps += b;
+            mixed += std::min(a, b);
         }
-        if (saved >= TENSOR_MIN_SAVING_MS) tbudget = tensor_budget(c, free_memory());
+        if (all_tensor <= mixed) std::fill(on_tensor.begin(), on_tensor.end(), 1);
+        if (std::min(all_tensor, mixed) < all_sweeps) tbudget = tensor_budget(c, free_memory());
         if (!tbudget) std::fill(on_tensor.begin(), on_tensor.end(), 0);
     }
     std::vector<uint64_t> all_cols(ncol.begin(), ncol.begin() + nb);   // what each bucket multiplies in all
@@ -1184,7 +1192,7 @@ void wl_close(wl_ctx* c) {
                        &c->bbitmap, &c->bsegcount, &c->boffsets, &c->boffs, &c->wcols, &c->wbuckets, &c->witems,
                        &c->wpart, &c->wdefs, &c->bacc, &c->bdef, &c->wkeys, &c->wcounts, &c->uacc, &c->udef,
                        &c->defs, &c->rowout, &c->prod, &c->windesc, &c->seglo, &c->work,
-                       &c->tb.desc, &c->tb.counts, &c->tb.tables, &c->tb.list, &c->tb.w, &c->tb.consts, &c->tb.ones,
+                       &c->tb.desc, &c->tb.counts, &c->tb.cursor, &c->tb.lab_seg, &c->tb.runs, &c->tb.segs, &c->tb.tables, &c->tb.list, &c->tb.w, &c->tb.consts, &c->tb.ones,
                        &c->tb.part, &c->tb.seg, &c->tb.win, &c->gprod, &c->gk };
     for (DevBuf* b : bufs) if (b->p) cudaFree(b->p);
     for (auto& e : c->ev) if (e) cudaEventDestroy(e);

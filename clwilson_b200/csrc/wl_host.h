@@ -116,7 +116,7 @@ inline int limb_width(uint64_t pmax_incl) {
 
 // Workspace of the tensor-core column products (wl_tensor_host.cu).
 struct TensorBufs {
-    DevBuf desc, counts, tables, list, w, consts, ones, part, seg, win;
+    DevBuf desc, counts, cursor, lab_seg, runs, segs, tables, list, w, consts, ones, part, seg, win;
 };
 
 struct wl_ctx {
@@ -180,10 +180,10 @@ int gen_test_primes(wl_ctx* c, const wl_range* ranges, size_t nr, std::vector<Ra
 // Workspace the tensor-core products may take with `free_bytes` of device
 // memory free; 0: too little, the sweeps run instead.
 size_t tensor_budget(wl_ctx* c, size_t free_bytes);
-// Modelled time that the tensor-core product saves over the sweeps for a bucket
-// of nrows rows over nsparse + ndense columns from index c0 on, in ms (negative:
-// the sweeps are faster).
-double tensor_saves(uint32_t nrows, int L, uint64_t T, uint64_t c0, uint64_t nsparse, uint64_t ndense);
+// Modelled times (ms) of the tensor-core product and of the sweeps for a bucket
+// of nrows rows over nsparse + ndense columns from index c0 on.
+void tensor_times(uint32_t nrows, int L, uint64_t T, uint64_t c0, uint64_t nsparse, uint64_t ndense, double* tensor,
+                  double* sweeps);
 // Multiplies each task's columns into its rows' accumulators (uacc), on the
 // main stream; rowmod must be set up.  Row indices are below nrows_total.
 int tensor_products(wl_ctx* c, std::vector<wl::TensorTask> tasks, uint32_t nrows_total, size_t budget);

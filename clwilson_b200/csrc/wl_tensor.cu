@@ -133,6 +133,106 @@ k_tensor_scatter(const TensorDesc* __restrict__ desc, uint32_t ntask, const uint
 }
 
 // ---------------------------------------------------------------------------
+// Layout: labels -> places in the list, lane runs, slots and segments.  One CTA
+// per task scans its labels 256 at a time; planned here rather than on the host
+// because a batch has hundreds of tasks of thousands of labels each (192 tasks:
+// 80 ms of host time, most of the call).
+// ---------------------------------------------------------------------------
+
+// Columns of a group of which none is above q: an eighth of them stays below 2^512
+// (k_tensor_build), so the group below 2^4096.
+__device__ __forceinline__ uint32_t group_columns(uint64_t q) {
+    const double k = 511.99 / log2((double)(q < 2 ? 2 : q) + 1.0);
+    return 8 * (uint32_t)fmin(k, (double)(TN_GMAX / 8));
+}
+
+struct LabelPlan { uint32_t n, g, longs, shorts; };
+
+// Columns of label (j, d) have v_q(T!) >= d 2^(wj), so q <= T / (d 2^(wj)) + 1.
+__device__ __forceinline__ LabelPlan plan_label(const TensorDesc& d, uint32_t l, uint32_t n, uint32_t g_all) {
+    LabelPlan p = { n, g_all, 0, 0 };
+    if (!n) return p;
+    const uint32_t dg = l & ((1u << d.w) - 1), j = l >> d.w;
+    const uint64_t q = (d.T >> (d.w * j)) / dg + 1;
+    if (q < d.q_max) p.g = group_columns(q);
+    const uint32_t ng = (n + p.g - 1) / p.g;
+    p.longs = ng / TN_LONG;
+    p.shorts = (ng % TN_LONG + TN_SHORT - 1) / TN_SHORT;
+    if (p.shorts * TN_SHORT >= TN_LONG) { ++p.longs; p.shorts = 0; }
+    return p;
+}
+
+// Exclusive prefix sum of v over the CTA's 256 threads, *total its sum.
+__device__ __forceinline__ uint32_t cta_scan(uint32_t v, uint32_t* total) {
+    __shared__ uint32_t ws[8];
+    const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    uint32_t incl = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t x = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= (uint32_t)o) incl += x;
+    }
+    __syncthreads();
+    if (lane == 31) ws[wid] = incl;
+    __syncthreads();
+    uint32_t before = 0, all = 0;
+#pragma unroll
+    for (uint32_t i = 0; i < 8; ++i) {
+        before += i < wid ? ws[i] : 0u;
+        all += ws[i];
+    }
+    *total = all;
+    return before + incl - v;
+}
+
+// FILL = 0: sizes only.  FILL = 1: the tables too.
+template <int FILL>
+__global__ void __launch_bounds__(256)
+k_tensor_layout(const TensorDesc* __restrict__ desc, const uint32_t* __restrict__ counts, TensorSize* __restrict__ size,
+                uint32_t* __restrict__ cursor, LaneRun* __restrict__ runs, FoldSeg* __restrict__ segs,
+                uint32_t* __restrict__ lab_seg) {
+    const TensorDesc d = desc[blockIdx.x];
+    const uint32_t labels = d.nwin << d.w, g_all = group_columns(d.q_max);
+    uint32_t entries = 0, longs = 0, shorts = 0, slots = 0, nseg = 0;
+    for (uint32_t l0 = 0; l0 < labels; l0 += 256) {
+        const uint32_t l = l0 + threadIdx.x;
+        const LabelPlan p = plan_label(d, l, l < labels ? counts[d.lab0 + l] : 0u, g_all);
+        uint32_t t_n, t_long, t_short, t_slot, t_seg;
+        const uint32_t at = entries + cta_scan(p.n, &t_n);
+        const uint32_t lo = longs + cta_scan(p.longs, &t_long), sh = shorts + cta_scan(p.shorts, &t_short);
+        // one slot per warp that the label's long runs touch, one per short run
+        const uint32_t nslot = p.shorts + (p.longs ? (lo + p.longs - 1) / 32 - lo / 32 + 1 : 0u);
+        const uint32_t sl = slots + cta_scan(nslot, &t_slot);
+        const uint32_t sg = nseg + cta_scan((nslot + TN_SEG - 1) / TN_SEG, &t_seg);
+        if (FILL && l < labels) {
+            const uint32_t start = d.list0 + at, end = start + p.n;
+            cursor[d.lab0 + l] = start;
+            lab_seg[d.lab_seg0 + l] = sg;
+            for (uint32_t k = 0; k < p.longs; ++k)
+                runs[d.long0 + lo + k] = { start + k * p.g * TN_LONG, end, p.g, sl + (lo + k) / 32 - lo / 32 };
+            const uint32_t s0 = sl + nslot - p.shorts, c0 = start + p.longs * p.g * TN_LONG;
+            for (uint32_t k = 0; k < p.shorts; ++k)
+                runs[d.short0 + sh + k] = { c0 + k * p.g * TN_SHORT, end, p.g, s0 + k };
+            for (uint32_t k = 0; k < nslot; k += TN_SEG)
+                segs[d.seg0 + sg + k / TN_SEG] = { sl + k, min(TN_SEG, nslot - k) };
+        }
+        entries += t_n;
+        longs += t_long;
+        shorts += t_short;
+        slots += t_slot;
+        nseg += t_seg;
+    }
+    if (FILL) {
+        if (threadIdx.x == 0) lab_seg[d.lab_seg0 + labels] = nseg;
+        // the last tiles' lanes without a run: groups of no column
+        for (uint32_t k = longs + threadIdx.x; k < d.nlong; k += 256) runs[d.long0 + k] = { 0, 0, 1, RUN_NONE };
+        for (uint32_t k = shorts + threadIdx.x; k < d.nshort; k += 256) runs[d.short0 + k] = { 0, 0, 1, RUN_NONE };
+    } else if (threadIdx.x == 0) {
+        size[blockIdx.x] = { entries, longs, shorts, slots, nseg };
+    }
+}
+
+// ---------------------------------------------------------------------------
 // Group products: one warp multiplies up to g columns into 128 limbs.  Each
 // lane multiplies its share of the columns serially (5 limbs), then five levels
 // of pairwise products in shared memory bring 32 shares to one number.  The
@@ -790,14 +890,13 @@ k_tensor_fold(const TensorDesc* __restrict__ desc, uint32_t ntask, const FoldSeg
 // One thread per (row, window j, block b of 32 digits): prod A_{j,d}^d over the
 // block's digits d = 32 b + o, as prod A^o (running products from the top digit
 // down) times (prod A)^(32 b).  Blocks keep the serial chain at about 80 products.
-// lab_seg[lab0 + l] .. lab_seg[lab0 + l + 1]: segments of label l (task-relative).
+// lab_seg[lab_seg0 + l] .. lab_seg[lab_seg0 + l + 1]: segments of label l (task-relative).
 template <int L>
 __global__ void __launch_bounds__(TF_THREADS)
 k_tensor_windows(const TensorDesc* __restrict__ desc, uint32_t ntask, const uint32_t* __restrict__ lab_seg,
                  const RowMod* __restrict__ mods, const uint4* __restrict__ ones,
                  const typename PartOf<L>::T* __restrict__ seg_part, typename PartOf<L>::T* __restrict__ win) {
-    const uint32_t ti = task_of_block(desc, ntask, blockIdx.x, &TensorDesc::row_blk0);
-    const TensorDesc& d = desc[ti];
+    const TensorDesc& d = desc[task_of_block(desc, ntask, blockIdx.x, &TensorDesc::row_blk0)];
     const uint32_t nb = (1u << d.w) / TN_DIGITS, j = blockIdx.y / nb, b = blockIdx.y % nb;
     const uint32_t r = (blockIdx.x - d.row_blk0) * TF_THREADS + threadIdx.x;
     if (j >= d.nwin || r >= d.nrows) return;
@@ -807,8 +906,7 @@ k_tensor_windows(const TensorDesc* __restrict__ desc, uint32_t ntask, const uint
 #pragma unroll
     for (int k = 0; k < L; ++k) n[k] = m.n[k];
     Res<L> S = res_of<L>(ones[row]), R = S;
-    // label tables of task ti are one longer than its labels
-    const uint32_t* ls = lab_seg + d.lab0 + ti + (j << d.w) + b * TN_DIGITS;
+    const uint32_t* ls = lab_seg + d.lab_seg0 + (j << d.w) + b * TN_DIGITS;
     bool any = false;
     for (int o = TN_DIGITS - 1; o >= 0; --o) {
         for (uint32_t s = ls[o]; s < ls[o + 1]; ++s) {
@@ -860,6 +958,13 @@ k_tensor_rows(const TensorDesc* __restrict__ desc, uint32_t ntask, const RowMod*
 void launch_tensor_count(const TensorDesc* d, uint32_t ntask, uint32_t nblocks, const uint32_t* cols, uint32_t* counts,
                          cudaStream_t st) {
     k_tensor_count<<<nblocks, 256, 0, st>>>(d, ntask, cols, counts);
+}
+void launch_tensor_size(const TensorDesc* d, uint32_t ntask, const uint32_t* counts, TensorSize* size, cudaStream_t st) {
+    k_tensor_layout<0><<<ntask, 256, 0, st>>>(d, counts, size, nullptr, nullptr, nullptr, nullptr);
+}
+void launch_tensor_layout(const TensorDesc* d, uint32_t ntask, const uint32_t* counts, uint32_t* cursor, LaneRun* runs,
+                          FoldSeg* segs, uint32_t* lab_seg, cudaStream_t st) {
+    k_tensor_layout<1><<<ntask, 256, 0, st>>>(d, counts, nullptr, cursor, runs, segs, lab_seg);
 }
 void launch_tensor_scatter(const TensorDesc* d, uint32_t ntask, uint32_t nblocks, const uint32_t* cols,
                            uint32_t* cursor, uint32_t* list, cudaStream_t st) {

@@ -37,14 +37,23 @@ struct TensorDesc {
     uint64_t seg_part0;  // first element of its segment products
     uint64_t win0;       // first element of its window products (a row of them per window and digit block)
     uint32_t c0, c1;
+    uint32_t q_max;      // no column is above it
     uint32_t row_begin, nrows, rows_pad;   // rows_pad: whole row tiles
     uint32_t w, nwin;    // digit width and count
     uint32_t lab0;       // first label (nwin << w of them)
+    uint32_t lab_seg0;   // first entry of its table of label segments (one longer than the labels)
     uint32_t blk0;       // first CTA of the digit sort
     uint32_t ct0;        // first row-constant tile
     uint32_t fold_blk0, row_blk0;   // first CTA of the segment fold / per-row kernels
     uint32_t seg0, nseg;
+    uint32_t list0;      // first list entry
+    uint32_t long0, nlong, short0, nshort;   // its lane runs of both lengths: first, padded count
 };
+// What a task takes, from its digit counts.
+struct TensorSize { uint32_t entries, longs, shorts, slots, segs; };
+// Groups per lane run: a label's groups go in runs of 32, the rest in runs of
+// 4, so that a label wastes about two groups however many it has.
+constexpr uint32_t TN_LONG = 32, TN_SHORT = 4;
 // A section of a task: 128-lane blocks of lane runs of the same length.
 struct TensorSec {
     uint32_t task;
@@ -66,6 +75,11 @@ struct TensorItem { uint32_t sec, tile, cb0, ncb; };
 
 void launch_tensor_count(const TensorDesc* d, uint32_t ntask, uint32_t nblocks, const uint32_t* cols, uint32_t* counts,
                          cudaStream_t st);
+// the tasks' sizes, from the counts
+void launch_tensor_size(const TensorDesc* d, uint32_t ntask, const uint32_t* counts, TensorSize* size, cudaStream_t st);
+// their list places (cursor), lane runs, label segments
+void launch_tensor_layout(const TensorDesc* d, uint32_t ntask, const uint32_t* counts, uint32_t* cursor, LaneRun* runs,
+                          FoldSeg* segs, uint32_t* lab_seg, cudaStream_t st);
 void launch_tensor_scatter(const TensorDesc* d, uint32_t ntask, uint32_t nblocks, const uint32_t* cols,
                            uint32_t* cursor, uint32_t* list, cudaStream_t st);
 // the group products of nmt group tiles, in the tiles' shared-memory image
