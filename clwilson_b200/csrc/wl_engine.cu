@@ -147,14 +147,8 @@ ColGroups col_groups(wl_ctx* c) {
 // the exponent -- that last 0.3 to 2.5 ms however few the rows are; the
 // tensor-core product's eight launches and its wait about 0.1.  Both measured on
 // calls of 15 to 3,600 rows at 1e5 to 2^62 (1e7, 61 rows: 0.92 against 0.27 ms;
-// 2^62, 30 rows, q < 2^20: 2.10 against 0.41).  WL_TENSOR=0 in the environment
-// turns the tensor-core product off, for comparisons.
+// 2^62, 30 rows, q < 2^20: 2.10 against 0.41).
 constexpr double SWEEP_CALL_MS = 0.4, TENSOR_CALL_MS = 0.1;
-static bool tensor_enabled() {
-    static const bool off = getenv("WL_TENSOR") && atoi(getenv("WL_TENSOR")) == 0;
-    return !off;
-}
-
 struct HostBucket {
     uint32_t range, type, L;
     uint64_t T;
@@ -617,17 +611,18 @@ static int run_ranges(wl_ctx* c, const wl_range* ranges, size_t nr, uint64_t qca
     size_t tbudget = 0;
     if (tensor_enabled()) {
         // all buckets on one path, or, where both have work, each on its faster one
-        double all_tensor = TENSOR_CALL_MS, all_sweeps = SWEEP_CALL_MS, mixed = TENSOR_CALL_MS + SWEEP_CALL_MS;
+        double all_tensor = TENSOR_CALL_MS, all_sweeps = SWEEP_CALL_MS, mixed = TENSOR_CALL_MS + SWEEP_CALL_MS,
+               entries = 0;
         for (size_t i = 0; i < nb; ++i) {
             double a, b;
-            tensor_times((uint32_t)hb[i].primes.size(), (int)hb[i].L, hb[i].T, cb_lo[i], ncol[i] - ndn[i], ndn[i], &a, &b);
+            entries += tensor_times((uint32_t)hb[i].primes.size(), (int)hb[i].L, hb[i].T, cb_lo[i], ncol[i] - ndn[i], ndn[i], &a, &b);
             on_tensor[i] = a < b;
             all_tensor += a;
             all_sweeps += b;
             mixed += std::min(a, b);
         }
         if (all_tensor <= mixed) std::fill(on_tensor.begin(), on_tensor.end(), 1);
-        if (std::min(all_tensor, mixed) < all_sweeps) tbudget = tensor_budget(c, free_memory());
+        if (std::min(all_tensor, mixed) < all_sweeps) tbudget = tensor_budget(c, entries, (double)nrows);
         if (!tbudget) std::fill(on_tensor.begin(), on_tensor.end(), 0);
     }
     std::vector<uint64_t> all_cols(ncol.begin(), ncol.begin() + nb);   // what each bucket multiplies in all
@@ -901,7 +896,7 @@ static int run_ranges(wl_ctx* c, const wl_range* ranges, size_t nr, uint64_t qca
     cg.record(c->ev[2], c->st);
     if (!tensor.empty()) {
         // planned from counts that the device makes, so outside the graph
-        RC(tensor_products(c, tensor, nrows, tbudget));
+        RC(tensor_products(c, tensor, { as<RowMod>(c->rowmod), as<uint4>(c->uacc), as<uint32_t>(c->work) + 6 }, tbudget));
         if (as_graph) RC(cg.begin(c->st));
     }
     size_t ioff = 0;

@@ -177,15 +177,21 @@ struct RangeState {
 // device); with allow_empty a range without primes is not an error.
 int gen_test_primes(wl_ctx* c, const wl_range* ranges, size_t nr, std::vector<RangeState>& rs,
                     std::vector<uint64_t>& tps, bool allow_empty = false);
-// Workspace the tensor-core products may take with `free_bytes` of device
-// memory free; 0: too little, the sweeps run instead.
-size_t tensor_budget(wl_ctx* c, size_t free_bytes);
+// WL_TENSOR=0 in the environment turns the tensor-core products off, for comparisons.
+inline bool tensor_enabled() {
+    static const bool off = getenv("WL_TENSOR") && atoi(getenv("WL_TENSOR")) == 0;
+    return !off;
+}
+// Workspace the tensor-core products may take for about `entries` list entries
+// and `rows` rows; 0: too little memory, the sweeps run instead.
+size_t tensor_budget(wl_ctx* c, double entries, double rows);
 // Modelled times (ms) of the tensor-core product and of the sweeps for a bucket
-// of nrows rows over nsparse + ndense columns from index c0 on.
-void tensor_times(uint32_t nrows, int L, uint64_t T, uint64_t c0, uint64_t nsparse, uint64_t ndense, double* tensor,
-                  double* sweeps);
-// Multiplies each task's columns into its rows' accumulators (uacc), on the
-// main stream; rowmod must be set up.  Row indices are below nrows_total.
-int tensor_products(wl_ctx* c, std::vector<wl::TensorTask> tasks, uint32_t nrows_total, size_t budget);
+// of nrows rows over nsparse + ndense columns from index c0 on; returns its list
+// entries.
+double tensor_times(uint32_t nrows, int L, uint64_t T, uint64_t c0, uint64_t nsparse, uint64_t ndense, double* tensor,
+                    double* sweeps);
+// Multiplies each task's columns into its rows' accumulators, on the main
+// stream (it waits once for the stream).
+int tensor_products(wl_ctx* c, std::vector<wl::TensorTask> tasks, const wl::TensorTarget& to, size_t budget);
 // results.txt value of one row (cl_wilson.cpp:872-898): 1 if it is a result line.
 int result_of(const wl_row& r, int32_t* value);

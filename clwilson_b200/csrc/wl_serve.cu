@@ -60,6 +60,7 @@ struct SBucket {
     // sweep, bend = key + 1; nroot sieving primes (67 .. sqrt(key)) for them
     uint64_t bpos = 0, bend = 0, key = 0;
     uint32_t nroot = 0;
+    double tcost = 0;                          // cells a column costs as a tensor-core product; 0: the sweeps are faster
     bool stop = false;                         // cancelled: no further chunks
     bool done() const { return pos >= ncols && bpos >= bend; }
     bool idle() const { return stop || done(); }
@@ -68,6 +69,11 @@ struct SBucket {
 constexpr uint64_t BIG_LO = 1ull << 32;   // first integer above the resident column table
 // cost of sieving one integer above 2^32, in cells of the sweep (measured on B200)
 constexpr double BIG_SIEVE_CELLS = 1.6;
+// seconds a cell of the step's budget stands for
+constexpr double CELL_SECONDS = 1.2e-12;
+// A chunk of a tensor-core product has at least this many columns: its labels
+// and launches cost as much as some ten thousand.
+constexpr uint64_t TENSOR_CHUNK = 65536;
 
 uint64_t isqrt_floor(uint64_t n) {
     uint64_t r = (uint64_t)std::sqrt((long double)n);
@@ -105,6 +111,8 @@ struct wl_server {
     uint64_t step_cells = 0;
     uint32_t shares = WL_SHARES_LEAST_WORK;
     DevBuf info, mods, acc, out, pbuckets, bdef, ipart;
+    DevBuf terr;                               // error word of the tensor-core products
+    size_t tbudget = 0;                        // workspace they may take (0: none, the sweeps run)
     // Two sets of a step's buffers: the scheduler plans and queues step k+1
     // into one set while step k still runs on the other, and completes step k
     // (its timing, the requests whose lift followed it) meanwhile.
@@ -113,6 +121,7 @@ struct wl_server {
         DevBuf bbitmap, bsegcount, boffs, bkeys, blos;   // columns above 2^32: bitmaps and their keys
         cudaEvent_t e0 = nullptr, e1 = nullptr;
         bool inflight = false;
+        bool tensor = false;                         // ran tensor-core products: their error word is read
         std::vector<SReq*> finishing;                // their lift runs right after this step
         uint32_t dirty_top = 1u << 30;               // device descriptors at or above: all nsplit = 0
     } slot[2];
@@ -341,6 +350,12 @@ static void serve_admit_batch(wl_server* s, const std::vector<SReq*>& cands, std
             b.bend = b.key >= BIG_LO ? b.key + 1 : BIG_LO;
             // column cache: cols[0 .. 17] = 2 .. 61, the presieve of k_sieve_big
             b.nroot = b.key >= BIG_LO && cnt[2 * nk + ki] > 18 ? (uint32_t)(cnt[2 * nk + ki] - 18) : 0;
+            b.tcost = 0;
+            if (s->tbudget && b.ncols) {
+                double ta, tw;
+                tensor_times(b.nrows, (int)b.L, a.T[t], 0, b.ncols - b.cdense, b.cdense, &ta, &tw);
+                if (ta < tw) b.tcost = ta * 1e-3 / CELL_SECONDS / (double)b.ncols;
+            }
             Bucket& d = s->pdesc[bid];
             memset(&d, 0, sizeof(d));
             d.T = a.T[t];
@@ -449,7 +464,8 @@ static int serve_step(wl_server* s) {
     wl_ctx* c = s->c;
     wl_server::Slot& sl = s->slot[s->cur];      // not in flight: the loop completes it first
     // kind 0: sparse columns of the resident table, 1: dense ones, 2: a chunk of
-    // the number line above 2^32 (integers [c0, c0 + len), sieved this step)
+    // the number line above 2^32 (integers [c0, c0 + len), sieved this step), 3:
+    // columns of the resident table as a tensor-core product
     struct Work { uint32_t bid; uint64_t c0, len; int kind; };
     std::vector<Work> work;
     // The step's descriptor table covers every slot a merge may meet (a merge
@@ -479,7 +495,9 @@ static int serve_step(wl_server* s) {
     // half floor, and equal shares gave longer ones.)
     auto work_left = [](const SBucket& b) {
         double r = 0;
-        if (b.pos < b.ncols) {
+        if (b.pos < b.ncols && b.tcost > 0) {
+            r += b.tcost * (double)(b.ncols - b.pos);
+        } else if (b.pos < b.ncols) {
             const uint64_t dl = b.pos < b.cdense ? b.cdense - b.pos : 0;
             const uint64_t sl = b.ncols - std::max(b.pos, b.cdense);
             r += (double)b.nrows * (5.0 * (double)dl + (double)sl);
@@ -521,7 +539,14 @@ static int serve_step(wl_server* s) {
         Work w;
         w.bid = bid;
         double per, cost;
-        if (b.pos < b.ncols) {
+        if (b.pos < b.ncols && b.tcost > 0) {
+            w.c0 = b.pos;
+            w.kind = 3;
+            w.len = std::min<uint64_t>(b.ncols - b.pos, std::max<uint64_t>((uint64_t)(share / b.tcost), TENSOR_CHUNK));
+            if (b.ncols - b.pos - w.len < w.len / 4) w.len = b.ncols - b.pos;
+            work.push_back(w);
+            continue;
+        } else if (b.pos < b.ncols) {
             w.c0 = b.pos;
             w.kind = b.pos < b.cdense ? 1 : 0;
             per = (double)b.nrows * (w.kind ? 5.0 : 1.0);
@@ -558,8 +583,21 @@ static int serve_step(wl_server* s) {
     uint32_t def_total = 0;
     std::vector<uint32_t> bucket_splits(top, 0);
     std::vector<uint64_t> bkeys, blos;
+    std::vector<TensorTask> tensor;
     for (const Work& w : work) {
         const SBucket& b = s->sb[w.bid];
+        if (w.kind == 3) {
+            TensorTask t;
+            t.T = s->pdesc[w.bid].T;
+            t.c0 = w.c0;
+            t.c1 = w.c0 + w.len;
+            t.row_begin = s->pdesc[w.bid].row_begin;
+            t.nrows = b.nrows;
+            t.L = (int)b.L;
+            t.q_max = (uint32_t)std::min<uint64_t>(b.key, BIG_LO - 1);
+            tensor.push_back(t);
+            continue;
+        }
         Bucket& x = sbk[w.bid];
         x = s->pdesc[w.bid];
         int rpt = 1;
@@ -639,6 +677,13 @@ static int serve_step(wl_server* s) {
         RC(ensure_step(s, sl.blos, (size_t)s->bucket_cap * 8));
     }
     cudaEventRecord(sl.e0, c->st);
+    if (!tensor.empty()) {
+        // waits for the step before it; its own kernels then run beside the planning below
+        const uint32_t before = c->launches;
+        RC(tensor_products(c, tensor, { as<RowMod>(s->mods), as<uint4>(s->acc), as<uint32_t>(s->terr) }, s->tbudget));
+        s->ws.launches += c->launches - before;
+        sl.tensor = true;
+    }
     CK(cudaMemcpyAsync(sl.sbuckets.p, sbk.data(), sbk.size() * sizeof(Bucket), cudaMemcpyHostToDevice, c->st));
     sl.dirty_top = top;
     CK(cudaMemcpyAsync(sl.items.p, all.data(), all.size() * sizeof(SweepItem), cudaMemcpyHostToDevice, c->st));
@@ -781,6 +826,13 @@ static void serve_complete(wl_server* s, wl_server::Slot& sl, int err = 0) {
     if (!sl.inflight) return;
     const double t = s->now_ms();
     if (!err && cudaEventSynchronize(sl.e1) != cudaSuccess) err = WL_ERR_CUDA;
+    if (!err && sl.tensor) {
+        uint32_t ran_out = 0;
+        if (cudaMemcpyAsync(&ran_out, s->terr.p, 4, cudaMemcpyDeviceToHost, s->c->st3) != cudaSuccess ||
+            cudaStreamSynchronize(s->c->st3) != cudaSuccess || ran_out)
+            err = WL_ERR_CUDA;
+    }
+    sl.tensor = false;
     if (!err) {
         float ms = 0;
         cudaEventElapsedTime(&ms, sl.e0, sl.e1);
@@ -923,16 +975,17 @@ int wl_server_open(const wl_server_opts* opts, wl_server** out) {
     if (ensure(s->info, (size_t)s->pool_cap * sizeof(RowInfo)) || ensure(s->mods, (size_t)s->pool_cap * sizeof(RowMod)) ||
         ensure(s->acc, (size_t)s->pool_cap * 16) || ensure(s->out, (size_t)s->pool_cap * sizeof(RowOut)) ||
         ensure(s->pbuckets, s->bucket_cap * sizeof(Bucket)) || ensure(s->bdef, s->bucket_cap * sizeof(Deficit)) ||
-        cudaEventCreate(&s->e0) != cudaSuccess || cudaEventCreate(&s->e1) != cudaSuccess ||
+        ensure(s->terr, 16) || cudaMemset(s->terr.p, 0, 16) != cudaSuccess || cudaEventCreate(&s->e0) != cudaSuccess || cudaEventCreate(&s->e1) != cudaSuccess ||
         cudaEventCreate(&s->slot[0].e0) != cudaSuccess || cudaEventCreate(&s->slot[0].e1) != cudaSuccess ||
         cudaEventCreate(&s->slot[1].e0) != cudaSuccess || cudaEventCreate(&s->slot[1].e1) != cudaSuccess) {
         cudaGetLastError();
-        DevBuf* bufs[] = { &s->info, &s->mods, &s->acc, &s->out, &s->pbuckets, &s->bdef };
+        DevBuf* bufs[] = { &s->info, &s->mods, &s->acc, &s->out, &s->pbuckets, &s->bdef, &s->terr };
         for (DevBuf* b : bufs) if (b->p) cudaFree(b->p);
         wl_close(s->c);
         delete s;
         return WL_ERR_NOMEM;
     }
+    if (tensor_enabled()) s->tbudget = tensor_budget(s->c, 1e9, 1e6);   // what a large call would take
     // the step buffers' pool, which keeps what is freed into it; each set of
     // step buffers starts at the size a step of the default budget takes
     // (about two rows of split products per thread of the sweep, a split
@@ -1085,7 +1138,7 @@ void wl_server_close(wl_server* s) {
     if (s->worker.joinable()) s->worker.join();
     cudaSetDevice(s->c->device);
     cudaStreamSynchronize(s->c->st);
-    DevBuf* bufs[] = { &s->info, &s->mods, &s->acc, &s->out, &s->pbuckets, &s->bdef, &s->ipart };
+    DevBuf* bufs[] = { &s->info, &s->mods, &s->acc, &s->out, &s->pbuckets, &s->bdef, &s->ipart, &s->terr };
     for (DevBuf* b : bufs) if (b->p) cudaFree(b->p);
     for (auto& sl : s->slot) {
         DevBuf* sb[] = { &sl.sbuckets, &sl.items, &sl.part, &sl.defs, &sl.bbitmap, &sl.bsegcount, &sl.boffs,

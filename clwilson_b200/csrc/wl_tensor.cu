@@ -495,7 +495,7 @@ k_tensor_consts(const TensorDesc* __restrict__ desc, uint32_t ntask, const RowMo
         for (int k = 0; k < L; ++k) n[k] = md.n[k];
         const Res<L> one = mont_one<L>(n);         // R mod n
         if (sg == 0)
-            ones[row] = make_uint4(one.w[0], one.w[1], L > 2 ? one.w[2 < L ? 2 : 0] : 0, L > 3 ? one.w[3 < L ? 3 : 0] : 0);
+            ones[tile * RT + r] = make_uint4(one.w[0], one.w[1], L > 2 ? one.w[2 < L ? 2 : 0] : 0, L > 3 ? one.w[3 < L ? 3 : 0] : 0);
         Res<L> m256 = one;                         // 256 R mod n
         for (int k = 0; k < 8; ++k) dbl_mod<L>(m256, n);
         // 2^(128 sg + 32) R = 2^(8 (16 sg) + 32 (L + 1)) mod n
@@ -775,7 +775,7 @@ k_tensor_gemm(const TensorDesc* __restrict__ desc, const TensorSec* __restrict__
         uint32_t t = 0;
         for (uint32_t cb = it.cb0; cb < it.cb0 + it.ncb && ok; ++cb) {
 #pragma unroll
-            for (uint32_t r = 0; r < RH; ++r) P[r] = res_of<L>(ones[r < live ? row0 + r : d.row_begin]);
+            for (uint32_t r = 0; r < RH; ++r) P[r] = res_of<L>(ones[(d.ct0 + it.tile) * RT + (r < live ? r0 + r : 0)]);
             for (uint32_t k = 0; k < tn; ++k, ++t) {
                 const uint32_t buf = t & 1;
                 ok = mbar_wait(bAccFull + 8 * buf, (t >> 1) & 1);
@@ -905,7 +905,7 @@ k_tensor_windows(const TensorDesc* __restrict__ desc, uint32_t ntask, const uint
     uint32_t n[L];
 #pragma unroll
     for (int k = 0; k < L; ++k) n[k] = m.n[k];
-    Res<L> S = res_of<L>(ones[row]), R = S;
+    Res<L> S = res_of<L>(ones[d.ct0 * tn_rows(L) + r]), R = S;
     const uint32_t* ls = lab_seg + d.lab_seg0 + (j << d.w) + b * TN_DIGITS;
     bool any = false;
     for (int o = TN_DIGITS - 1; o >= 0; --o) {

@@ -30,6 +30,14 @@ constexpr uint32_t TN_DIGITS = 32;      // digits per block of the window produc
 constexpr uint32_t TN_SEG = 64;         // slots per segment of the label fold
 __host__ __device__ constexpr uint32_t tn_rows(int L) { return TN_N / (4u * (uint32_t)L); }
 
+// Where the rows live: their moduli, the accumulators to multiply into, and a
+// word that a kernel sets when one of its waits runs out.
+struct TensorTarget {
+    const RowMod* mods;
+    uint4* acc;
+    uint32_t* err;
+};
+
 // Device descriptor of a task.
 struct TensorDesc {
     uint64_t T;
@@ -85,6 +93,7 @@ void launch_tensor_scatter(const TensorDesc* d, uint32_t ntask, uint32_t nblocks
 // the group products of nmt group tiles, in the tiles' shared-memory image
 void launch_tensor_build(const TensorSec* sec, uint32_t nsec, uint32_t nmt, const LaneRun* lr, const uint32_t* list,
                          uint8_t* w, cudaStream_t st);
+// ones: R mod n of every row of every tile
 void launch_tensor_consts(int L, const TensorDesc* d, uint32_t ntask, uint32_t ntiles, const RowMod* mods, uint8_t* consts,
                           uint4* ones, cudaStream_t st);
 int launch_tensor_gemm(int L, uint32_t nitems, const TensorDesc* d, const TensorSec* sec, const TensorItem* items,

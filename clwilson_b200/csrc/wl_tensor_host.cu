@@ -82,7 +82,7 @@ struct Tables {
 
 class Products {
 public:
-    Products(wl_ctx* c, size_t budget) : c(c), tb(c->tb) {
+    Products(wl_ctx* c, const TensorTarget& to, size_t budget) : c(c), tb(c->tb), to(to) {
         lim.entries = std::min<double>((double)budget / 2 / 9.0, (double)(1u << 25));
         lim.part = std::min<double>((double)budget / 4, 256e6);
         lim.consts = std::min<double>((double)budget / 4, 128e6);
@@ -93,6 +93,7 @@ public:
 private:
     wl_ctx* c;
     TensorBufs& tb;
+    TensorTarget to;
     Limits lim;
     std::vector<TensorTask> tasks;
     // the current wave
@@ -293,6 +294,7 @@ int Products::chunk(const TensorTask* ts, size_t i0, size_t i1) {
         }
         Tables tab;
         const size_t o_desc = tab.add(dc), o_sec = tab.add(secs), o_item = tab.add(items);
+        RC(ensure(tb.ones, (size_t)ntile * rt * 16 + 16));
         RC(ensure(tb.tables, tab.bytes.size()));
         RC(ensure(tb.seg, seg * esz + 16));
         RC(ensure(tb.win, win * esz + 16));
@@ -303,7 +305,7 @@ int Products::chunk(const TensorTask* ts, size_t i0, size_t i1) {
         const TensorDesc* dd = (const TensorDesc*)(base + o_desc);
         const TensorSec* ds = (const TensorSec*)(base + o_sec);
         const LaneRun* dr = as<LaneRun>(tb.runs);
-        const RowMod* mods = as<RowMod>(c->rowmod);
+        const RowMod* mods = to.mods;
         if (first) {
             launch_tensor_layout(dd, nt, as<uint32_t>(tb.counts), as<uint32_t>(tb.cursor), as<LaneRun>(tb.runs),
                                  as<FoldSeg>(tb.segs), as<uint32_t>(tb.lab_seg), st);
@@ -314,11 +316,11 @@ int Products::chunk(const TensorTask* ts, size_t i0, size_t i1) {
         launch_tensor_consts(L, dd, nt, ntile, mods, as<uint8_t>(tb.consts), as<uint4>(tb.ones), st);
         if (launch_tensor_gemm(L, (uint32_t)items.size(), dd, ds, (const TensorItem*)(base + o_item), dr, mods,
                                as<uint8_t>(tb.w), as<uint8_t>(tb.consts), as<uint4>(tb.ones), tb.part.p,
-                               as<uint32_t>(c->work) + 6, st))
+                               to.err, st))
             return WL_ERR_CUDA;
         launch_tensor_fold(L, dd, nt, fold_blk, as<FoldSeg>(tb.segs), mods, tb.part.p, tb.seg.p, st);
         launch_tensor_combine(L, dd, nt, row_blk, max_blocks, as<uint32_t>(tb.lab_seg), mods, as<uint4>(tb.ones),
-                              tb.seg.p, tb.win.p, as<uint4>(c->uacc), st);
+                              tb.seg.p, tb.win.p, to.acc, st);
         CK(cudaGetLastError());
         c->launches += 5;
         first = false;
@@ -332,10 +334,15 @@ int Products::chunk(const TensorTask* ts, size_t i0, size_t i1) {
 // The least free memory the tensor-core path takes on, and the most workspace it plans for.
 static constexpr size_t TENSOR_MIN_BUDGET = 1ull << 30, TENSOR_MAX_BUDGET = 2ull << 30;
 
-size_t tensor_budget(wl_ctx* c, size_t free_bytes) {
+size_t tensor_budget(wl_ctx* c, double entries, double rows) {
+    // lists, group products, constants and products of a small call, several
+    // times over: the query of the free memory would cost it a sixth of its time
+    if (16.0 * entries + 16384.0 * rows <= 192e6) return TENSOR_MIN_BUDGET;
     const TensorBufs& b = c->tb;
     const size_t held = b.list.cap + b.w.cap + b.consts.cap + b.part.cap + b.seg.cap + b.win.cap;
-    const size_t budget = std::min(TENSOR_MAX_BUDGET, (free_bytes + held) / 2);
+    size_t free_b = 0, total_b = 0;
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) { cudaGetLastError(); free_b = 8ull << 30; }
+    const size_t budget = std::min(TENSOR_MAX_BUDGET, (free_b + held) / 2);
     return budget < TENSOR_MIN_BUDGET ? 0 : budget;
 }
 
@@ -347,12 +354,12 @@ size_t tensor_budget(wl_ctx* c, size_t free_bytes) {
 //   entry: 36 (3.1 ms for 8.7e7 entries at 4 limbs); per row tile: 0.8 (17.0 ms
 //   for 2.2e10 at 2 limbs)
 //   cell: 0.68 / 1.0 / 1.35; dense column: 8 / 11 / 14.6 (L = 2 / 3 / 4)
-void tensor_times(uint32_t nrows, int L, uint64_t T, uint64_t c0, uint64_t nsparse, uint64_t ndense, double* tensor,
-                  double* sweeps) {
+double tensor_times(uint32_t nrows, int L, uint64_t T, uint64_t c0, uint64_t nsparse, uint64_t ndense, double* tensor,
+                    double* sweeps) {
     static const double cell[3] = { 0.68, 1.0, 1.35 }, dense[3] = { 8.0, 11.0, 14.6 };
     const uint64_t ncols = nsparse + ndense;
     *tensor = *sweeps = 0;
-    if (!ncols || !nrows) return;
+    if (!ncols || !nrows) return 0;
     TensorTask t = {};
     t.T = T;
     t.c0 = c0;
@@ -362,12 +369,12 @@ void tensor_times(uint32_t nrows, int L, uint64_t T, uint64_t c0, uint64_t nspar
     const double entries = (double)ncols * entries_per_column(t, w) + 150.0 * (double)(1u << w);
     *tensor = entries * (36.0 + 0.8 * row_tiles_of(nrows, L)) * 1e-9;
     *sweeps = ((double)nrows + 16.0) * (cell[L - 2] * (double)nsparse + dense[L - 2] * (double)ndense) * 1e-9;
+    return entries;
 }
 
-int tensor_products(wl_ctx* c, std::vector<TensorTask> tasks, uint32_t nrows_total, size_t budget) {
+int tensor_products(wl_ctx* c, std::vector<TensorTask> tasks, const TensorTarget& to, size_t budget) {
     std::stable_sort(tasks.begin(), tasks.end(), [](const TensorTask& a, const TensorTask& b) { return a.L < b.L; });
-    RC(ensure(c->tb.ones, (size_t)nrows_total * 16 + 16));
-    Products p(c, budget);
+    Products p(c, to, budget);
     for (const TensorTask& t : tasks) p.add(t);
     return p.run();
 }
