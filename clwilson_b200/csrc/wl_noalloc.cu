@@ -58,10 +58,10 @@ __global__ void k_noalloc_clear() {
     *reinterpret_cast<uint32_t*>(g_noalloc_scratch + OFF_FLAG) = 0;
 }
 
-// One sweep's items: `tiles` row tiles of `nsplit` splits from split0 on,
+// One sweep's items: `tiles` row tiles of its splits from split0 on,
 // 256 / tps splits to an item when the rows fit one narrow tile.
 struct ItemPlan {
-    uint32_t tps, split0, nsplit, nitems;
+    uint32_t tps, split0, tiles, nitems;
 };
 
 __device__ wl::SweepItem plan_item(const ItemPlan& p, uint32_t i) {
@@ -69,8 +69,9 @@ __device__ wl::SweepItem plan_item(const ItemPlan& p, uint32_t i) {
     it.bucket = 0;
     it.tps = p.tps;
     if (p.tps == 256) {
-        it.row0 = (i / p.nsplit) * 256;
-        it.split0 = p.split0 + i % p.nsplit;
+        // all row tiles of a split before the next: the first splits fold most often and start first
+        it.row0 = (i % p.tiles) * 256;
+        it.split0 = p.split0 + i / p.tiles;
     } else {
         it.row0 = 0;
         it.split0 = p.split0 + i * (256 / p.tps);
@@ -239,12 +240,21 @@ extern "C" int wl_column_product_noalloc(const uint64_t* primes, uint32_t nrows,
         sd = std::max<uint32_t>(sd, 1);
         if (ns <= 0) sd = nsplit;
         else if (sd >= nsplit) sd = nsplit > 1 ? nsplit - 1 : 0;
+        // the prefix-fold sweep in whole waves of four CTAs per SM (a split and row
+        // tile each), the splits left over to the dense sweep, which runs before it
+        // and would otherwise leave most of the SMs idle
+        const uint32_t tiles = (nrows + 255) / 256, slots = 4 * (uint32_t)sms, ss = nsplit - sd;
+        if (nrows >= 256 && sd && ss * tiles >= slots) {
+            const uint32_t whole = ss * tiles / slots * slots / tiles;
+            sd = std::max(sd, std::min(nsplit - whole, (uint32_t)(nd / 128.0)));
+            nsplit = sd + whole;
+        }
     }
     auto plan = [&](uint32_t split0, uint32_t n, uint32_t min_tps) {
-        ItemPlan p = { 256, split0, n, 0 };
+        ItemPlan p = { 256, split0, (nrows + 255) / 256, 0 };
         if (n == 0) return p;
         if (nrows >= 256) {
-            p.nitems = ((nrows + 255) / 256) * n;
+            p.nitems = p.tiles * n;
         } else {
             p.tps = min_tps;
             while (p.tps < nrows) p.tps <<= 1;
