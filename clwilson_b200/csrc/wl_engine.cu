@@ -149,6 +149,7 @@ ColGroups col_groups(wl_ctx* c) {
 // calls of 15 to 3,600 rows at 1e5 to 2^62 (1e7, 61 rows: 0.92 against 0.27 ms;
 // 2^62, 30 rows, q < 2^20: 2.10 against 0.41).
 constexpr double SWEEP_CALL_MS = 0.4, TENSOR_CALL_MS = 0.1;
+constexpr uint64_t TENSOR_TAIL_MIN = 100000000;
 struct HostBucket {
     uint32_t range, type, L;
     uint64_t T;
@@ -809,16 +810,25 @@ static int run_ranges(wl_ctx* c, const wl_range* ranges, size_t nr, uint64_t qca
     // consecutive-integer tail (full search only): row r has it_count chunks of
     // K integers starting at T+1; the items themselves are derived on the device
     uint64_t n_items = 0, K = 1;
+    std::vector<TensorTail> tails;      // buckets whose tail runs on the tensor cores
     out.tail = 0;
     if (full) {
         uint64_t Wt = 0;
         for (uint32_t r = 0; r < nrows; ++r) Wt += ri[r].Tp - db[ri[r].bucket].T;
         out.tail = Wt;
+        // long tails go to the tensor cores with the columns (tensor_tails): four
+        // launches, worth it from some 10^8 cells (0.07 ms of k_iterate)
+        if (tbudget && Wt >= TENSOR_TAIL_MIN) {
+            for (const Bucket& b : db)
+                if (ri[b.row_begin + b.nrows - 1].Tp < TAIL_MAX) tails.push_back({ b.T, b.row_begin, b.nrows, b.L });
+        }
         const double tgt_items = (double)c->sms * 2048.0 * 2.0;
         K = std::max<uint64_t>(1024, (uint64_t)std::ceil((double)Wt / tgt_items));
         K = std::min<uint64_t>(K, 1u << 30);
+        std::vector<char> tailed(db.size(), 0);
+        for (const TensorTail& t : tails) tailed[ri[t.row_begin].bucket] = 1;
         for (uint32_t r = 0; r < nrows; ++r) {
-            const uint64_t len = ri[r].Tp - db[ri[r].bucket].T;
+            const uint64_t len = tailed[ri[r].bucket] ? 0 : ri[r].Tp - db[ri[r].bucket].T;
             ri[r].it_begin = (uint32_t)n_items;
             ri[r].it_count = (uint32_t)((len + K - 1) / K);
             n_items += ri[r].it_count;
@@ -875,7 +885,8 @@ static int run_ranges(wl_ctx* c, const wl_range* ranges, size_t nr, uint64_t qca
     // columns above 2^32, whose windows are planned from device counts)
     ChainGraph cg;
     const bool as_graph = graph && !init && !big_need;
-    if (as_graph && tensor.empty()) RC(cg.begin(c->st));
+    const TensorTarget target = { as<RowMod>(c->rowmod), as<uint4>(c->uacc), as<uint32_t>(c->work) + 6 };
+    if (as_graph && tensor.empty() && tails.empty()) RC(cg.begin(c->st));
     launch_acc_init(nrows, (uint32_t)db.size(), as<uint4>(c->uacc), as<Deficit>(c->udef), c->st);
     c->launches++;
     if (init) {
@@ -894,9 +905,10 @@ static int run_ranges(wl_ctx* c, const wl_range* ranges, size_t nr, uint64_t qca
     c->launches++;
     CK(cudaEventRecord(c->rows_ready, c->st));
     cg.record(c->ev[2], c->st);
-    if (!tensor.empty()) {
+    if (!tensor.empty() || !tails.empty()) {
         // planned from counts that the device makes, so outside the graph
-        RC(tensor_products(c, tensor, { as<RowMod>(c->rowmod), as<uint4>(c->uacc), as<uint32_t>(c->work) + 6 }, tbudget));
+        if (!tensor.empty()) RC(tensor_products(c, tensor, target, tbudget));
+        if (!tails.empty()) RC(tensor_tails(c, tails, ri, target));
         if (as_graph) RC(cg.begin(c->st));
     }
     size_t ioff = 0;

@@ -193,5 +193,9 @@ double tensor_times(uint32_t nrows, int L, uint64_t T, uint64_t c0, uint64_t nsp
 // Multiplies each task's columns into its rows' accumulators, on the main
 // stream (it waits once for the stream).
 int tensor_products(wl_ctx* c, std::vector<wl::TensorTask> tasks, const wl::TensorTarget& to, size_t budget);
+// Multiplies the rows' consecutive-integer tails T+1 .. Tp into their
+// accumulators, on the main stream; c->rowinfo holds the rows ri.
+int tensor_tails(wl_ctx* c, const std::vector<wl::TensorTail>& tails, const std::vector<wl::RowInfo>& ri,
+                 const wl::TensorTarget& to);
 // results.txt value of one row (cl_wilson.cpp:872-898): 1 if it is a result line.
 int result_of(const wl_row& r, int32_t* value);

@@ -395,51 +395,37 @@ __device__ __forceinline__ void build_high(const uint32_t* x, uint32_t* part, ui
     carry_up(out, carry, li, lp);
 }
 
-__global__ void __launch_bounds__(TB_WARPS * 32)
-k_tensor_build(const TensorSec* __restrict__ secs, uint32_t nsec, const LaneRun* __restrict__ lr,
-               const uint32_t* __restrict__ list, uint8_t* __restrict__ w) {
-    __shared__ __align__(16) uint32_t sx[TB_WARPS][TB_X];
-    __shared__ __align__(16) uint32_t sp[TB_WARPS][TB_P];
-    const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    constexpr uint32_t PER_TILE = TN_M / TB_WARPS;      // CTAs per group tile
-    const uint32_t mt = blockIdx.x / PER_TILE;
-    const uint32_t m = (blockIdx.x % PER_TILE) * TB_WARPS + wid;      // lane of the tile
-    const TensorSec sec = secs[task_of_block(secs, nsec, mt, &TensorSec::mt0)];
-    const uint32_t local = mt - sec.mt0, cb = local / sec.tn, t = local % sec.tn;
-    const LaneRun run = lr[sec.run0 + cb * TN_M + m];
-    const uint64_t beg = (uint64_t)run.start + (uint64_t)t * run.g;
-    const uint32_t n = beg < run.end ? (uint32_t)min((uint64_t)run.g, run.end - beg) : 0u;
-    // limbs 4 lane .. 4 lane + 3: bytes 16 lane .. of the group, chunk lane % 8 of
-    // block lane / 8 (128-byte swizzle: chunk ^ (row % 8))
+// The place of a lane's four limbs of group m of group tile mt: limbs 4 lane ..
+// 4 lane + 3 are bytes 16 lane .. of the group, chunk lane % 8 of block lane / 8
+// (128-byte swizzle: chunk ^ (row % 8)).
+__device__ __forceinline__ uint4* group_place(uint8_t* w, uint32_t mt, uint32_t m, uint32_t lane) {
     const uint32_t kb = lane >> 3, ch = lane & 7;
-    uint8_t* dst = w + (((uint64_t)mt * TN_KB + kb) * TN_M + m) * 128 + ((ch ^ (m & 7)) << 4);
-    if (n == 0) {                                      // no column: the product is 1
-        *reinterpret_cast<uint4*>(dst) = make_uint4(lane == 0 ? 1u : 0u, 0u, 0u, 0u);
-        return;
-    }
-    uint32_t* x = sx[wid];
-    uint32_t* p = sp[wid];
+    return reinterpret_cast<uint4*>(w + (((uint64_t)mt * TN_KB + kb) * TN_M + m) * 128 + ((ch ^ (m & 7)) << 4));
+}
 
-    // the lane's share: a quarter of its eighth of the columns
-    {
-        uint32_t a[5] = { 1, 0, 0, 0, 0 };
-        const uint32_t e = lane >> 2, q0 = n * e / 8, nq = n * (e + 1) / 8 - q0;
-        const uint32_t k0 = q0 + nq * (lane & 3) / 4, k1 = q0 + nq * ((lane & 3) + 1) / 4;
-        for (uint32_t k = k0; k < k1; ++k) {
-            const uint32_t q = list[beg + k];
-            uint64_t carry = 0;
+// The lane's part [k0, k1) of a group's n numbers: a quarter of its eighth.
+__device__ __forceinline__ void share_of(uint32_t n, uint32_t lane, uint32_t* k0, uint32_t* k1) {
+    const uint32_t e = lane >> 2, q0 = n * e / 8, nq = n * (e + 1) / 8 - q0;
+    *k0 = q0 + nq * (lane & 3) / 4;
+    *k1 = q0 + nq * ((lane & 3) + 1) / 4;
+}
+
+__device__ __forceinline__ void share_times(uint32_t (&a)[5], uint32_t q) {
+    uint64_t carry = 0;
 #pragma unroll
-            for (int i = 0; i < 5; ++i) {
-                const uint64_t v = (uint64_t)a[i] * q + carry;
-                a[i] = (uint32_t)v;
-                carry = v >> 32;
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < 5; ++i) x[lane * 5 + i] = a[i];
+    for (int i = 0; i < 5; ++i) {
+        const uint64_t v = (uint64_t)a[i] * q + carry;
+        a[i] = (uint32_t)v;
+        carry = v >> 32;
     }
+}
+
+// The product of the warp's 32 shares; the lane's four limbs come back in out.
+__device__ __forceinline__ void build_tree(const uint32_t (&a)[5], uint32_t* x, uint32_t* p, uint32_t lane, uint32_t (&out)[4]) {
+#pragma unroll
+    for (int i = 0; i < 5; ++i) x[lane * 5 + i] = a[i];
     __syncwarp();
-    uint32_t out[4], top;
+    uint32_t top;
     build_low<4>(x, p, p + 176, p + 352, lane, out, &top);     // 5 x 5 limbs -> 9
     {
         const uint32_t ob = (lane >> 1) * 9, li = lane & 1;
@@ -459,7 +445,71 @@ k_tensor_build(const TensorSec* __restrict__ secs, uint32_t nsec, const LaneRun*
     *xv = make_uint4(out[0], out[1], out[2], out[3]);
     __syncwarp();
     build_high<64, 8, 16>(x, p, lane, out);
-    *reinterpret_cast<uint4*>(dst) = make_uint4(out[0], out[1], out[2], out[3]);
+}
+
+__global__ void __launch_bounds__(TB_WARPS * 32)
+k_tensor_build(const TensorSec* __restrict__ secs, uint32_t nsec, const LaneRun* __restrict__ lr,
+               const uint32_t* __restrict__ list, uint8_t* __restrict__ w) {
+    __shared__ __align__(16) uint32_t sx[TB_WARPS][TB_X];
+    __shared__ __align__(16) uint32_t sp[TB_WARPS][TB_P];
+    const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    constexpr uint32_t PER_TILE = TN_M / TB_WARPS;      // CTAs per group tile
+    const uint32_t mt = blockIdx.x / PER_TILE;
+    const uint32_t m = (blockIdx.x % PER_TILE) * TB_WARPS + wid;      // lane of the tile
+    const TensorSec sec = secs[task_of_block(secs, nsec, mt, &TensorSec::mt0)];
+    const uint32_t local = mt - sec.mt0, cb = local / sec.tn, t = local % sec.tn;
+    const LaneRun run = lr[sec.run0 + cb * TN_M + m];
+    const uint64_t beg = (uint64_t)run.start + (uint64_t)t * run.g;
+    const uint32_t n = beg < run.end ? (uint32_t)min((uint64_t)run.g, run.end - beg) : 0u;
+    uint4* dst = group_place(w, mt, m, lane);
+    if (n == 0) {                                      // no column: the product is 1
+        *dst = make_uint4(lane == 0 ? 1u : 0u, 0u, 0u, 0u);
+        return;
+    }
+    uint32_t a[5] = { 1, 0, 0, 0, 0 }, k0, k1, out[4];
+    share_of(n, lane, &k0, &k1);
+    for (uint32_t k = k0; k < k1; ++k) share_times(a, list[beg + k]);
+    build_tree(a, sx[wid], sp[wid], lane, out);
+    *dst = make_uint4(out[0], out[1], out[2], out[3]);
+}
+
+// Groups of consecutive integers: group j = 128 tile + m of a bucket's tail holds
+// T + 1 + j g .. T + (j + 1) g.
+__global__ void __launch_bounds__(TB_WARPS * 32)
+k_tensor_tail_build(const TensorDesc* __restrict__ desc, const TensorSec* __restrict__ secs, uint32_t nsec,
+                    uint8_t* __restrict__ w) {
+    __shared__ __align__(16) uint32_t sx[TB_WARPS][TB_X];
+    __shared__ __align__(16) uint32_t sp[TB_WARPS][TB_P];
+    const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    constexpr uint32_t PER_TILE = TN_M / TB_WARPS;
+    const uint32_t mt = blockIdx.x / PER_TILE;
+    const uint32_t m = (blockIdx.x % PER_TILE) * TB_WARPS + wid;
+    const TensorSec sec = secs[task_of_block(secs, nsec, mt, &TensorSec::mt0)];
+    const uint64_t first = desc[sec.task].T + 1 + ((uint64_t)(mt - sec.mt0) * TN_M + m) * sec.g;
+    uint32_t a[5] = { 1, 0, 0, 0, 0 }, k0, k1, out[4];
+    share_of(sec.g, lane, &k0, &k1);
+    for (uint32_t k = k0; k < k1; ++k) {
+        const uint64_t N = first + k;
+        const uint32_t hi = (uint32_t)(N >> 32);
+        if (hi == 0) {
+            share_times(a, (uint32_t)N);
+        } else {                                       // a lo + (a hi) 2^32
+            uint32_t b[5];
+#pragma unroll
+            for (int i = 0; i < 5; ++i) b[i] = a[i];
+            share_times(a, (uint32_t)N);
+            share_times(b, hi);
+            uint64_t c = 0;
+#pragma unroll
+            for (int i = 1; i < 5; ++i) {
+                c += (uint64_t)a[i] + b[i - 1];
+                a[i] = (uint32_t)c;
+                c >>= 32;
+            }
+        }
+    }
+    build_tree(a, sx[wid], sp[wid], lane, out);
+    *group_place(w, mt, m, lane) = make_uint4(out[0], out[1], out[2], out[3]);
 }
 
 // ---------------------------------------------------------------------------
@@ -674,10 +724,16 @@ __device__ __forceinline__ Res<L> res_of(const uint4& v) {
 // for the item; group tiles stream through 16 KB stages; the accumulator is
 // double-buffered (2 x 256 tensor-memory columns), so that the epilogue of one
 // tile runs beside the next tile's product.
-template <int L>
+//
+// TAIL = 1: the groups are those of a bucket's consecutive-integer tail, lane
+// after lane, and a row leaves out those past its own end (info); an item is a
+// row tile with the group tiles that some row of it needs, and each warp writes
+// one product per row.
+template <int L, int TAIL>
 __global__ void __launch_bounds__(TG_THREADS, 1)
 k_tensor_gemm(const TensorDesc* __restrict__ desc, const TensorSec* __restrict__ secs,
-              const TensorItem* __restrict__ items, const LaneRun* __restrict__ lr, const RowMod* __restrict__ mods,
+              const TensorItem* __restrict__ items, const LaneRun* __restrict__ lr, const RowInfo* __restrict__ info,
+              const RowMod* __restrict__ mods,
               const uint8_t* __restrict__ w, const uint8_t* __restrict__ consts, const uint4* __restrict__ ones,
               typename PartOf<L>::T* __restrict__ part, uint32_t* __restrict__ err) {
     extern __shared__ uint8_t smem_raw[];
@@ -691,7 +747,7 @@ k_tensor_gemm(const TensorDesc* __restrict__ desc, const TensorSec* __restrict__
     const TensorItem it = items[blockIdx.x];
     const TensorSec sec = secs[it.sec];
     const TensorDesc& d = desc[sec.task];
-    const uint32_t tn = sec.tn, ntiles = it.ncb * tn;
+    const uint32_t tn = TAIL ? it.ncb : sec.tn, ncb = TAIL ? 1 : it.ncb, ntiles = ncb * tn;
     if (threadIdx.x == 0) {
         for (uint32_t s = 0; s < TG_STAGES; ++s) { mbar_init(bFull + 8 * s, 1); mbar_init(bEmpty + 8 * s, 1); }
         mbar_init(bConst, 1);
@@ -771,9 +827,15 @@ k_tensor_gemm(const TensorDesc* __restrict__ desc, const TensorSec* __restrict__
             for (int k = 0; k < L; ++k) n[r][k] = m.n[k];
             ninv[r] = m.ninv;
         }
+        uint32_t ends[TAIL ? RH : 1];              // groups of each row
+        if (TAIL) {
+#pragma unroll
+            for (uint32_t r = 0; r < RH; ++r)
+                ends[TAIL ? r : 0] = r < live ? (uint32_t)((info[row0 + r].Tp - d.T) / sec.g) : 0u;
+        }
         const uint32_t taddr = tmem + (quarter << 21) + r0 * 4 * L;
         uint32_t t = 0;
-        for (uint32_t cb = it.cb0; cb < it.cb0 + it.ncb && ok; ++cb) {
+        for (uint32_t cb = it.cb0; cb < it.cb0 + ncb && ok; ++cb) {
 #pragma unroll
             for (uint32_t r = 0; r < RH; ++r) P[r] = res_of<L>(ones[(d.ct0 + it.tile) * RT + (r < live ? r0 + r : 0)]);
             for (uint32_t k = 0; k < tn; ++k, ++t) {
@@ -795,16 +857,24 @@ k_tensor_gemm(const TensorDesc* __restrict__ desc, const TensorSec* __restrict__
 #pragma unroll
                         for (int j = 0; j < L; ++j) tmem_ld4(D[(r + 1) & 1][j], ta + nr * 4 * L + 4 * j);
                     }
-                    fold_digits<L>(P[r], D[r & 1], n[r], ninv[r]);
+                    if (TAIL) {
+                        Res<L> Q = P[r];
+                        fold_digits<L>(Q, D[r & 1], n[r], ninv[r]);
+                        const bool take = k * TN_M + quarter * 32 + lane < ends[TAIL ? r : 0];
+#pragma unroll
+                        for (int j = 0; j < L; ++j) P[r].w[j] = take ? Q.w[j] : P[r].w[j];
+                    } else {
+                        fold_digits<L>(P[r], D[r & 1], n[r], ninv[r]);
+                    }
                 }
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
                 if (lane == 0) mbar_arrive(bAccEmpty + 8 * buf);
             }
             if (!ok) break;
-            const uint32_t slot = lr[sec.run0 + cb * TN_M + quarter * 32 + lane].slot;
+            const uint32_t slot = TAIL ? quarter : lr[sec.run0 + cb * TN_M + quarter * 32 + lane].slot;
             bool write = slot != RUN_NONE;
-            if (sec.reduce) {
+            if (TAIL || sec.reduce) {
                 // lanes of one label lie side by side: the first of them collects
                 // their product (segmented reduction over the warp)
 #pragma unroll 1
@@ -951,6 +1021,51 @@ k_tensor_rows(const TensorDesc* __restrict__ desc, uint32_t ntask, const RowMod*
     acc[row] = make_uint4(A.w[0], A.w[1], L > 2 ? A.w[2 < L ? 2 : 0] : 0, L > 3 ? A.w[3 < L ? 3 : 0] : 0);
 }
 
+// The rest of a row's tail, fewer than g integers after its last whole group, one
+// cell each; then acc *= that, the four products of the groups, and the power of
+// two that the cells took out.
+template <int L>
+__global__ void __launch_bounds__(TF_THREADS)
+k_tensor_tail_rows(const TensorDesc* __restrict__ desc, const TensorSec* __restrict__ secs, uint32_t ntask,
+                   const RowInfo* __restrict__ info, const RowMod* __restrict__ mods, const uint4* __restrict__ ones,
+                   const typename PartOf<L>::T* __restrict__ part, uint4* __restrict__ acc) {
+    const uint32_t ti = task_of_block(desc, ntask, blockIdx.x, &TensorDesc::row_blk0);
+    const TensorDesc& d = desc[ti];
+    const uint32_t r = (blockIdx.x - d.row_blk0) * TF_THREADS + threadIdx.x;
+    if (r >= d.nrows) return;
+    const uint32_t row = d.row_begin + r;
+    const RowMod m = mods[row];
+    uint32_t n[L];
+#pragma unroll
+    for (int k = 0; k < L; ++k) n[k] = m.n[k];
+    const uint64_t Tp = info[row].Tp, len = Tp - d.T, g = secs[ti].g, whole = len / g * g;
+    const Res<L> one = res_of<L>(ones[d.ct0 * tn_rows(L) + r]);
+    Res<L> X = one;
+    uint32_t bits = 0;
+    for (uint64_t N = d.T + whole + 1; N <= Tp; ++N) {
+        if (N < 0x80000000ull) {
+            cell_w<L>(X, (uint32_t)N, n, m.ninv);
+            bits += 32;
+        } else {
+            cell64<L>(X, N, n, m.ninv);
+            bits += 64;
+        }
+    }
+    Res<L> two = one;
+    dbl_mod<L>(two, n);
+    X = mont_mul<L>(X, mont_pow<L>(two, (u128)bits, one, n, m.ninv), n, m.ninv);
+    if (whole) {
+#pragma unroll 1
+        for (uint32_t k = 0; k < TAIL_SLOTS; ++k) {
+            Res<L> y;
+            part_unpack(part[d.part0 + (uint64_t)k * d.rows_pad + r], y);
+            X = mont_mul<L>(X, y, n, m.ninv);
+        }
+    }
+    const Res<L> A = mont_mul<L>(res_of<L>(acc[row]), X, n, m.ninv);
+    acc[row] = make_uint4(A.w[0], A.w[1], L > 2 ? A.w[2 < L ? 2 : 0] : 0, L > 3 ? A.w[3 < L ? 3 : 0] : 0);
+}
+
 // ---------------------------------------------------------------------------
 // launch wrappers
 // ---------------------------------------------------------------------------
@@ -986,21 +1101,47 @@ void launch_tensor_consts(int L, const TensorDesc* d, uint32_t ntask, uint32_t n
     else if (L == 3) consts_l<3>(d, ntask, ntiles, mods, consts, ones, st);
     else consts_l<4>(d, ntask, ntiles, mods, consts, ones, st);
 }
-template <int L>
+template <int L, int TAIL>
 static int gemm_l(uint32_t nitems, const TensorDesc* d, const TensorSec* sec, const TensorItem* items, const LaneRun* lr,
-                  const RowMod* mods, const uint8_t* w, const uint8_t* consts, const uint4* ones, void* part, uint32_t* err, cudaStream_t st) {
-    if (cudaFuncSetAttribute(k_tensor_gemm<L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TG_SMEM) != cudaSuccess)
+                  const RowInfo* info, const RowMod* mods, const uint8_t* w, const uint8_t* consts, const uint4* ones,
+                  void* part, uint32_t* err, cudaStream_t st) {
+    if (cudaFuncSetAttribute(k_tensor_gemm<L, TAIL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TG_SMEM) !=
+        cudaSuccess)
         return -1;
-    k_tensor_gemm<L><<<nitems, TG_THREADS, TG_SMEM, st>>>(d, sec, items, lr, mods, w, consts, ones,
-                                                          (typename PartOf<L>::T*)part, err);
+    k_tensor_gemm<L, TAIL><<<nitems, TG_THREADS, TG_SMEM, st>>>(d, sec, items, lr, info, mods, w, consts, ones,
+                                                                (typename PartOf<L>::T*)part, err);
     return 0;
 }
 int launch_tensor_gemm(int L, uint32_t nitems, const TensorDesc* d, const TensorSec* sec, const TensorItem* items,
-                       const LaneRun* lr, const RowMod* mods, const uint8_t* w, const uint8_t* consts, const uint4* ones, void* part, uint32_t* err,
-                       cudaStream_t st) {
-    if (L == 2) return gemm_l<2>(nitems, d, sec, items, lr, mods, w, consts, ones, part, err, st);
-    if (L == 3) return gemm_l<3>(nitems, d, sec, items, lr, mods, w, consts, ones, part, err, st);
-    return gemm_l<4>(nitems, d, sec, items, lr, mods, w, consts, ones, part, err, st);
+                       const LaneRun* lr, const RowMod* mods, const uint8_t* w, const uint8_t* consts,
+                       const uint4* ones, void* part, uint32_t* err, cudaStream_t st) {
+    if (L == 2) return gemm_l<2, 0>(nitems, d, sec, items, lr, nullptr, mods, w, consts, ones, part, err, st);
+    if (L == 3) return gemm_l<3, 0>(nitems, d, sec, items, lr, nullptr, mods, w, consts, ones, part, err, st);
+    return gemm_l<4, 0>(nitems, d, sec, items, lr, nullptr, mods, w, consts, ones, part, err, st);
+}
+void launch_tensor_tail_build(const TensorDesc* d, const TensorSec* sec, uint32_t nsec, uint32_t nmt, uint8_t* w,
+                              cudaStream_t st) {
+    k_tensor_tail_build<<<nmt * (TN_M / TB_WARPS), TB_WARPS * 32, 0, st>>>(d, sec, nsec, w);
+}
+int launch_tensor_tail_gemm(int L, uint32_t nitems, const TensorDesc* d, const TensorSec* sec, const TensorItem* items,
+                            const RowInfo* info, const RowMod* mods, const uint8_t* w, const uint8_t* consts,
+                            const uint4* ones, void* part, uint32_t* err, cudaStream_t st) {
+    if (L == 2) return gemm_l<2, 1>(nitems, d, sec, items, nullptr, info, mods, w, consts, ones, part, err, st);
+    if (L == 3) return gemm_l<3, 1>(nitems, d, sec, items, nullptr, info, mods, w, consts, ones, part, err, st);
+    return gemm_l<4, 1>(nitems, d, sec, items, nullptr, info, mods, w, consts, ones, part, err, st);
+}
+template <int L>
+static void tail_rows_l(const TensorDesc* d, const TensorSec* sec, uint32_t ntask, uint32_t nblocks, const RowInfo* info,
+                        const RowMod* mods, const uint4* ones, const void* part, uint4* acc, cudaStream_t st) {
+    k_tensor_tail_rows<L><<<nblocks, TF_THREADS, 0, st>>>(d, sec, ntask, info, mods, ones,
+                                                          (const typename PartOf<L>::T*)part, acc);
+}
+void launch_tensor_tail_rows(int L, const TensorDesc* d, const TensorSec* sec, uint32_t ntask, uint32_t nblocks,
+                             const RowInfo* info, const RowMod* mods, const uint4* ones, const void* part, uint4* acc,
+                             cudaStream_t st) {
+    if (L == 2) tail_rows_l<2>(d, sec, ntask, nblocks, info, mods, ones, part, acc, st);
+    else if (L == 3) tail_rows_l<3>(d, sec, ntask, nblocks, info, mods, ones, part, acc, st);
+    else tail_rows_l<4>(d, sec, ntask, nblocks, info, mods, ones, part, acc, st);
 }
 template <int L>
 static void fold_l(const TensorDesc* d, uint32_t ntask, uint32_t nblocks, const FoldSeg* segs, const RowMod* mods,

@@ -69,7 +69,7 @@ struct TensorSec {
     uint32_t mt0;        // first group tile
     uint32_t run0;       // first lane run
     uint32_t reduce;     // products of lanes with the same slot are multiplied before they are written
-    uint32_t pad;
+    uint32_t g;          // tails: integers per group
 };
 // A lane run: tn consecutive groups of one label's list, one after another in
 // one lane of the accumulator.  Group t covers list[start + t*g .. +g), cut at
@@ -78,6 +78,14 @@ struct LaneRun { uint32_t start, end, g, slot; };
 constexpr uint32_t RUN_NONE = 0xFFFFFFFFu;
 // Consecutive slots of one label, for the label fold.
 struct FoldSeg { uint32_t slot0, n; };
+// The consecutive-integer tails of a bucket's rows, T+1 .. Tp per row: groups of
+// `g` integers, group j the integers T + 1 + j g .., shared by all rows; a row
+// takes the first (Tp - T) / g of them here and the rest, fewer than g, one by one.
+struct TensorTail { uint64_t T; uint32_t row_begin, nrows, L; };
+// The largest integer a group may hold: a lane's share of a group's integers stays
+// below 2^160 up to 44 bits.
+constexpr uint64_t TAIL_MAX = 1ull << 44;
+constexpr uint32_t TAIL_SLOTS = 4;     // products per row: one from each warp quarter
 // One CTA's work: 128-lane blocks [cb0, cb0 + ncb) of a section against row tile `tile` of its task.
 struct TensorItem { uint32_t sec, tile, cb0, ncb; };
 
@@ -100,6 +108,17 @@ int launch_tensor_gemm(int L, uint32_t nitems, const TensorDesc* d, const Tensor
                        const LaneRun* lr, const RowMod* mods,
                        const uint8_t* w, const uint8_t* consts, const uint4* ones, void* part, uint32_t* err,
                        cudaStream_t st);
+// tails: group products, the matrix product with each row's own number of groups
+// (items: cb0 = 0, ncb = group tiles), and the rest of each row's integers with
+// the product into acc
+void launch_tensor_tail_build(const TensorDesc* d, const TensorSec* sec, uint32_t nsec, uint32_t nmt, uint8_t* w,
+                              cudaStream_t st);
+int launch_tensor_tail_gemm(int L, uint32_t nitems, const TensorDesc* d, const TensorSec* sec, const TensorItem* items,
+                            const RowInfo* info, const RowMod* mods, const uint8_t* w, const uint8_t* consts,
+                            const uint4* ones, void* part, uint32_t* err, cudaStream_t st);
+void launch_tensor_tail_rows(int L, const TensorDesc* d, const TensorSec* sec, uint32_t ntask, uint32_t nblocks,
+                             const RowInfo* info, const RowMod* mods, const uint4* ones, const void* part, uint4* acc,
+                             cudaStream_t st);
 void launch_tensor_fold(int L, const TensorDesc* d, uint32_t ntask, uint32_t nblocks, const FoldSeg* segs,
                         const RowMod* mods, const void* part, void* seg_part, cudaStream_t st);
 void launch_tensor_combine(int L, const TensorDesc* d, uint32_t ntask, uint32_t nblocks, uint32_t max_blocks,

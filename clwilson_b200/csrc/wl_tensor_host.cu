@@ -378,3 +378,80 @@ int tensor_products(wl_ctx* c, std::vector<TensorTask> tasks, const TensorTarget
     for (const TensorTask& t : tasks) p.add(t);
     return p.run();
 }
+
+// The tails of buckets of one limb width, a slab of rows at a time: row tiles
+// need whole group tiles only up to their last row's end (rows are in ascending
+// p, so ascending Tp).
+int tensor_tails(wl_ctx* c, const std::vector<TensorTail>& tails, const std::vector<RowInfo>& ri, const TensorTarget& to) {
+    cudaStream_t st = c->st;
+    TensorBufs& tb = c->tb;
+    for (size_t i0 = 0; i0 < tails.size();) {
+        const int L = (int)tails[i0].L;
+        const uint32_t rt = tn_rows(L);
+        std::vector<TensorDesc> dc;
+        std::vector<TensorSec> secs;
+        std::vector<TensorItem> items;
+        uint32_t ntile = 0, nmt = 0, row_blk = 0;
+        uint64_t part = 0;
+        size_t i1 = i0;
+        // as many tails as keep the constants within 128 MB and the groups within as much
+        for (; i1 < tails.size() && (int)tails[i1].L == L; ++i1) {
+            const TensorTail& t = tails[i1];
+            const uint64_t last = ri[t.row_begin + t.nrows - 1].Tp;
+            const double k = 511.99 / std::log2((double)last + 2.0);
+            const uint32_t g = 8 * (uint32_t)std::min<double>(k, (double)TN_GMAX / 8), tiles = row_tiles_of(t.nrows, L);
+            const uint64_t mts = ((last - t.T) / g + TN_M - 1) / TN_M;
+            if (i1 > i0 && (ntile + tiles > 1024 || nmt + mts > 2048)) break;
+            TensorDesc d;
+            memset(&d, 0, sizeof(d));
+            d.T = t.T;
+            d.row_begin = t.row_begin;
+            d.nrows = t.nrows;
+            d.rows_pad = tiles * rt;
+            d.ct0 = ntile;
+            d.row_blk0 = row_blk;
+            d.part0 = part;
+            const uint32_t s = (uint32_t)secs.size();
+            secs.push_back({ s, 0, nmt, 0, 1, g });
+            for (uint32_t r = 0; r < tiles; ++r) {
+                const uint32_t lr = std::min(t.nrows, (r + 1) * rt) - 1;
+                const uint64_t need = (ri[t.row_begin + lr].Tp - t.T) / g;
+                if (need) items.push_back({ s, r, 0, (uint32_t)((need + TN_M - 1) / TN_M) });
+            }
+            dc.push_back(d);
+            ntile += tiles;
+            nmt += (uint32_t)mts;
+            row_blk += (t.nrows + 127) / 128;
+            part += (uint64_t)TAIL_SLOTS * d.rows_pad;
+        }
+        // the longest tails first
+        std::stable_sort(items.begin(), items.end(),
+                         [](const TensorItem& a, const TensorItem& b) { return a.ncb > b.ncb; });
+        Tables tab;
+        const size_t o_desc = tab.add(dc), o_sec = tab.add(secs), o_item = tab.add(items);
+        RC(ensure(tb.tables, tab.bytes.size()));
+        RC(ensure(tb.consts, (size_t)ntile * TN_N * TN_K + 16));
+        RC(ensure(tb.ones, (size_t)ntile * rt * 16 + 16));
+        RC(ensure(tb.part, part * (L == 2 ? 8 : 16) + 16));
+        RC(ensure(tb.w, (size_t)nmt * TN_M * TN_K + 16));
+        CK(cudaMemcpyAsync(tb.tables.p, tab.bytes.data(), tab.bytes.size(), cudaMemcpyHostToDevice, st));
+        c->h2d += tab.bytes.size();
+        uint8_t* base = as<uint8_t>(tb.tables);
+        const TensorDesc* dd = (const TensorDesc*)(base + o_desc);
+        const TensorSec* ds = (const TensorSec*)(base + o_sec);
+        const uint32_t nt = (uint32_t)dc.size();
+        launch_tensor_consts(L, dd, nt, ntile, to.mods, as<uint8_t>(tb.consts), as<uint4>(tb.ones), st);
+        if (nmt) launch_tensor_tail_build(dd, ds, nt, nmt, as<uint8_t>(tb.w), st);
+        if (!items.empty() &&
+            launch_tensor_tail_gemm(L, (uint32_t)items.size(), dd, ds, (const TensorItem*)(base + o_item),
+                                    as<RowInfo>(c->rowinfo), to.mods, as<uint8_t>(tb.w), as<uint8_t>(tb.consts),
+                                    as<uint4>(tb.ones), tb.part.p, to.err, st))
+            return WL_ERR_CUDA;
+        launch_tensor_tail_rows(L, dd, ds, nt, row_blk, as<RowInfo>(c->rowinfo), to.mods, as<uint4>(tb.ones), tb.part.p,
+                                to.acc, st);
+        CK(cudaGetLastError());
+        c->launches += 4;
+        i0 = i1;
+    }
+    return 0;
+}

@@ -42,13 +42,26 @@ def test_capped_products(engine, lo, hi, qcap, nsample):
     _same(rows, want, sel)
 
 
-@pytest.mark.parametrize("lo,hi,nsample", [(3 * 10**6, 3 * 10**6 + 60000, 0), (3 * 10**8, 3 * 10**8 + 50000, 12)])
+# the last two have tails of 10^8 integers and more, whose groups run on the
+# tensor cores too: at 2 limbs, and with integers on both sides of 2^31
+@pytest.mark.parametrize("lo,hi,nsample", [(3 * 10**6, 3 * 10**6 + 60000, 0), (3 * 10**8, 3 * 10**8 + 50000, 12),
+                                           (10**8, 10**8 + 400000, 16), (2**32 - 10**5, 2**32 + 150000, 6)])
 def test_full_search(engine, lo, hi, nsample):
     rows, st = engine.rows(lo, hi)
     assert (rows["status"] == 0).all() and (rows["rem"] == 0).all()
     sel = np.linspace(0, len(rows) - 1, nsample).astype(np.uint32) if nsample else np.arange(len(rows), dtype=np.uint32)
     want, _ = oracle.search(lo, hi, rows=sel)
     _same(rows, want, sel, ("p", "s0", "s1", "rem", "quot"))
+
+
+@pytest.mark.parametrize("lo,hi", [(2**33 + 2 * 10**8, 2**33 + 2 * 10**8 + 120000)])
+def test_long_tail_equals_short_one(engine, lo, hi):
+    # integers past 2^32 in the tail.  T_p! does not depend on where its range
+    # starts: the last primes alone have a short tail, which runs cell by cell
+    rows, _ = engine.rows(lo, hi)
+    last, st = engine.rows(hi - 3000, hi)
+    assert (rows["status"] == 0).all() and st.tail_steps < 10**8
+    _same(rows[-len(last):], last, np.arange(len(last)), ("p", "s0", "s1", "rem", "quot"))
 
 
 def test_resumed_products(engine):
