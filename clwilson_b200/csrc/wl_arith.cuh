@@ -518,17 +518,51 @@ __device__ __forceinline__ uint64_t isqrt64(uint64_t n) {
     return x;
 }
 
+// floor(t / q) for t < 2^62, 2 <= q < 2^32, with inv = 1.0 / q: the double
+// product is off by t 2^-52 / q at most, so one correction from the remainder
+// (below 2^43, exact as a double) leaves it off by one at most.
+__host__ __device__ __forceinline__ uint64_t quot_inv(uint64_t t, uint32_t q, double inv) {
+    uint64_t e = (uint64_t)((double)t * inv);
+    int64_t r = (int64_t)(t - e * q);
+    if (t >> 52) {
+        const int64_t c = (int64_t)((double)r * inv);
+        e += (uint64_t)c;
+        r -= c * (int64_t)q;
+    }
+    if (r < 0) { --e; r += q; }
+    if (r < 0) { --e; r += q; }
+    if (r >= (int64_t)q) { ++e; r -= q; }
+    if (r >= (int64_t)q) ++e;
+    return e;
+}
+
 // Exponent of the prime q in T!: sum over k of floor(T / q^k) (Legendre's
 // formula; the reference's getPower, cl_wilson.cpp:1293-1313).  The terms come
-// as running quotients, floor(T / q^k) = floor(floor(T / q^(k-1)) / q), so a
-// term costs one division, and once a quotient and q fit 32 bits that division
-// is a 32-bit one (a 64-bit division costs several times as many multiplies).
+// as running quotients, floor(T / q^k) = floor(floor(T / q^(k-1)) / q): 32-bit
+// divisions where T fits, else products with the double 1/q (a 64-bit integer
+// division is some hundred instructions).
 __host__ __device__ __forceinline__ uint64_t legendre(uint64_t T, uint64_t q) {
-    uint64_t t = T / q, e = 0;
+    uint64_t e = 0;
+    if ((T >> 32) == 0) {
+        if (q >> 32) return 0;
+        uint32_t t = (uint32_t)T / (uint32_t)q;
+        while (t) {
+            e += t;
+            if (t < (uint32_t)q) break;                 // the next term is zero
+            t /= (uint32_t)q;
+        }
+        return e;
+    }
+    if (q >> 32) {
+        for (uint64_t t = T / q; t; t /= q) e += t;
+        return e;
+    }
+    const double inv = 1.0 / (double)q;
+    uint64_t t = quot_inv(T, (uint32_t)q, inv);
     while (t) {
         e += t;
-        if (t < q) break;                           // the next term is zero
-        t = ((t | q) >> 32) == 0 ? (uint64_t)((uint32_t)t / (uint32_t)q) : t / q;
+        if (t < q) break;
+        t = (t >> 32) ? quot_inv(t, (uint32_t)q, inv) : (uint64_t)((uint32_t)t / (uint32_t)q);
     }
     return e;
 }

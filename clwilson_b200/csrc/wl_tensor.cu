@@ -78,13 +78,19 @@ k_tensor_count(const TensorDesc* __restrict__ desc, uint32_t ntask, const uint32
     __syncthreads();
     const uint32_t b0 = d.c0 + (blockIdx.x - d.blk0) * TN_COLS_PER_BLOCK;
     const uint32_t b1 = min(d.c1, b0 + TN_COLS_PER_BLOCK);
-    for (uint32_t k = b0; k < b1; k += blockDim.x) {
-        const uint32_t c = k + threadIdx.x;
-        const bool in = c < b1;
-        const uint64_t e = in ? legendre(d.T, cols[c]) : 0;
+    // four columns at a time, so that their loads and divisions overlap
+    for (uint32_t k = b0 + threadIdx.x; k - threadIdx.x < b1; k += 4 * 256) {
+        uint64_t e[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) e[i] = k + 256 * i < b1 ? legendre(d.T, cols[k + 256 * i]) : 0;
         for (uint32_t j = 0; j < d.nwin; ++j) {
-            const uint32_t dg = (uint32_t)(e >> (d.w * j)) & mask;
-            warp_count(h, (j << d.w) | dg, in && dg != 0);
+            if (!__any_sync(0xffffffffu, (e[0] | e[1] | e[2] | e[3]) != 0)) break;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const uint32_t dg = (uint32_t)e[i] & mask;
+                warp_count(h, (j << d.w) | dg, dg != 0);
+                e[i] >>= d.w;
+            }
         }
     }
     __syncthreads();
@@ -93,41 +99,45 @@ k_tensor_count(const TensorDesc* __restrict__ desc, uint32_t ntask, const uint32
 }
 
 // cursor[label] starts at the label's place in `list`.  The order inside a
-// label depends on the order of the CTAs; its product does not.
+// label depends on the order of the CTAs; its product does not.  One digit at a
+// time: a column's slot among the CTA's columns of its label is counted once and
+// stays in a register until the CTA has its place in the list (counting again
+// for the write-out cost a third of the kernel: 0.58 ms for 5e7 columns).
 __global__ void __launch_bounds__(256)
 k_tensor_scatter(const TensorDesc* __restrict__ desc, uint32_t ntask, const uint32_t* __restrict__ cols,
                  uint32_t* __restrict__ cursor, uint32_t* __restrict__ list) {
-    __shared__ uint32_t h[TN_LABELS];
-    __shared__ uint64_t se[TN_COLS_PER_BLOCK];
-    const TensorDesc d = desc[task_of_block(desc, ntask, blockIdx.x, &TensorDesc::blk0)];
-    const uint32_t nlab = d.nwin << d.w, mask = (1u << d.w) - 1;
-    for (uint32_t i = threadIdx.x; i < nlab; i += blockDim.x) h[i] = 0;
-    __syncthreads();
-    const uint32_t b0 = d.c0 + (blockIdx.x - d.blk0) * TN_COLS_PER_BLOCK;
-    const uint32_t b1 = min(d.c1, b0 + TN_COLS_PER_BLOCK);
-    for (uint32_t k = b0; k < b1; k += blockDim.x) {
-        const uint32_t c = k + threadIdx.x;
-        const bool in = c < b1;
-        const uint64_t e = in ? legendre(d.T, cols[c]) : 0;
-        se[k - b0 + threadIdx.x] = e;
-        for (uint32_t j = 0; j < d.nwin; ++j) {
-            const uint32_t dg = (uint32_t)(e >> (d.w * j)) & mask;
-            warp_count(h, (j << d.w) | dg, in && dg != 0);
+    constexpr int PER = TN_COLS_PER_BLOCK / TN_SCATTER / 256;
+    __shared__ uint32_t h[1u << TN_WMAX];
+    const TensorDesc d = desc[task_of_block(desc, ntask, blockIdx.x / TN_SCATTER, &TensorDesc::blk0)];
+    const uint32_t nd = 1u << d.w, mask = nd - 1;
+    const uint32_t b0 = d.c0 + (blockIdx.x - d.blk0 * TN_SCATTER) * (256 * PER) + threadIdx.x;
+    const uint32_t b1 = d.c1;
+    uint64_t e[PER];
+#pragma unroll
+    for (int k = 0; k < PER; ++k) e[k] = b0 + 256 * k < b1 ? legendre(d.T, cols[b0 + 256 * k]) : 0;
+    for (uint32_t j = 0; j < d.nwin; ++j) {
+        uint64_t any = 0;
+#pragma unroll
+        for (int k = 0; k < PER; ++k) any |= e[k];
+        if (!__syncthreads_or(any != 0)) break;            // no digit left
+        for (uint32_t i = threadIdx.x; i < nd; i += 256) h[i] = 0;
+        __syncthreads();
+        uint32_t rank[PER];
+#pragma unroll
+        for (int k = 0; k < PER; ++k) {
+            const uint32_t dg = (uint32_t)e[k] & mask;
+            rank[k] = warp_count(h, dg, dg != 0);
         }
-    }
-    __syncthreads();
-    for (uint32_t i = threadIdx.x; i < nlab; i += blockDim.x)
-        if (h[i]) h[i] = atomicAdd(&cursor[d.lab0 + i], h[i]);
-    __syncthreads();
-    for (uint32_t k = b0; k < b1; k += blockDim.x) {
-        const uint32_t c = k + threadIdx.x;
-        const bool in = c < b1;
-        const uint32_t q = in ? cols[c] : 0;
-        const uint64_t e = se[k - b0 + threadIdx.x];
-        for (uint32_t j = 0; j < d.nwin; ++j) {
-            const uint32_t dg = (uint32_t)(e >> (d.w * j)) & mask;
-            const uint32_t pos = warp_count(h, (j << d.w) | dg, in && dg != 0);
-            if (in && dg != 0) list[pos] = q;
+        __syncthreads();
+        uint32_t* cur = cursor + d.lab0 + (j << d.w);
+        for (uint32_t i = threadIdx.x; i < nd; i += 256)
+            if (h[i]) h[i] = atomicAdd(&cur[i], h[i]);
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < PER; ++k) {
+            const uint32_t dg = (uint32_t)e[k] & mask;
+            if (dg) list[h[dg] + rank[k]] = cols[b0 + 256 * k];
+            e[k] >>= d.w;
         }
     }
 }
@@ -1083,7 +1093,7 @@ void launch_tensor_layout(const TensorDesc* d, uint32_t ntask, const uint32_t* c
 }
 void launch_tensor_scatter(const TensorDesc* d, uint32_t ntask, uint32_t nblocks, const uint32_t* cols,
                            uint32_t* cursor, uint32_t* list, cudaStream_t st) {
-    k_tensor_scatter<<<nblocks, 256, 0, st>>>(d, ntask, cols, cursor, list);
+    k_tensor_scatter<<<nblocks * TN_SCATTER, 256, 0, st>>>(d, ntask, cols, cursor, list);
 }
 void launch_tensor_build(const TensorSec* sec, uint32_t nsec, uint32_t nmt, const LaneRun* lr, const uint32_t* list,
                          uint8_t* w, cudaStream_t st) {

@@ -25,6 +25,8 @@ constexpr uint32_t TN_M = 128;          // groups per tile (tensor memory lanes)
 constexpr uint32_t TN_N = 256;          // row digits per tile: TN_N / (4L) rows
 constexpr uint32_t TN_GMAX = 512;       // columns per group at most
 constexpr uint32_t TN_COLS_PER_BLOCK = 4096;   // columns per CTA of the digit sort
+constexpr uint32_t TN_SCATTER = 2;      // CTAs of the write-out per CTA of the count
+constexpr uint32_t TN_WMAX = 9;         // bits of a digit at most
 constexpr uint32_t TN_LABELS = 4096;    // digit labels of a task at most
 constexpr uint32_t TN_DIGITS = 32;      // digits per block of the window products
 constexpr uint32_t TN_SEG = 64;         // slots per segment of the label fold
