@@ -126,7 +126,8 @@ assert ROW_DTYPE.itemsize == ctypes.sizeof(_Row)
 
 # exported symbols of include/wilson.h
 SYMBOLS = ("wl_open", "wl_close", "wl_strerror", "wl_stream", "wl_check_range", "wl_search", "wl_rows",
-           "wl_batch", "wl_rows_from", "wl_search_from", "wl_rows_product", "wl_drop_columns", "wl_parse_uint64",
+           "wl_batch", "wl_rows_from", "wl_search_from", "wl_rows_product", "wl_rows_product_parts",
+           "wl_drop_columns", "wl_parse_uint64",
            "wl_probe",
            "wl_column_product_noalloc", "wl_get_tuning", "wl_set_tuning", "wl_autotune",
            "wl_server_open", "wl_server_submit", "wl_server_poll", "wl_server_wait", "wl_server_results",
@@ -170,6 +171,8 @@ def load_library(path: str = LIB_PATH):
     L.wl_search_from.restype = ctypes.c_int
     L.wl_rows_product.argtypes = [vp, sz, vp, sz, vp, vp]
     L.wl_rows_product.restype = ctypes.c_int
+    L.wl_rows_product_parts.argtypes = [vp, sz, vp, sz, vp, vp]
+    L.wl_rows_product_parts.restype = ctypes.c_int
     L.wl_parse_uint64.argtypes = [ctypes.POINTER(u64), ctypes.c_char_p, u64, u64]
     L.wl_parse_uint64.restype = ctypes.c_int
     L.wl_drop_columns.argtypes = [vp]
@@ -425,19 +428,19 @@ class Engine:
             p = rows_parts[0]["p"]
         p = np.ascontiguousarray(p, dtype=np.uint64)
         n = p.size
-        digits = np.empty((len(parts), n, 2), dtype=np.uint64)
-        for k, x in enumerate(parts):
+        digits = []                                    # each part's digits in an array of their own
+        for x in parts:
             if x.dtype.names:
                 if not np.array_equal(x["p"], p):
                     raise ValueError("rows_product: the parts hold different primes")
-                digits[k, :, 0] = x["s0"]
-                digits[k, :, 1] = x["s1"]
+                digits.append(np.stack([x["s0"], x["s1"]], axis=1))
             else:
                 if x.shape != (n, 2):
                     raise ValueError("rows_product: a digit part must have shape (%d, 2)" % n)
-                digits[k] = x
+                digits.append(np.ascontiguousarray(x, dtype=np.uint64))
+        ptrs = (ctypes.c_void_p * len(parts))(*[d.ctypes.data for d in digits])
         out = np.zeros((max(n, 1), 2), dtype=np.uint64)
-        rc = self._L.wl_rows_product(self._ctx, n, p.ctypes.data, len(parts), digits.ctypes.data, out.ctypes.data)
+        rc = self._L.wl_rows_product_parts(self._ctx, n, p.ctypes.data, len(parts), ptrs, out.ctypes.data)
         if rc:
             raise WilsonError(rc, "wl_rows_product")
         rows = np.zeros(n, dtype=ROW_DTYPE)

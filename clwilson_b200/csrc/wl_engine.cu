@@ -1279,31 +1279,41 @@ int wl_search_from(wl_ctx* c, uint64_t pmin, uint64_t pmax, uint64_t q_lo, const
     return summarize(ro, 1, true, nullptr, results, cap, nullptr, stats);
 }
 
-int wl_rows_product(wl_ctx* c, size_t n, const uint64_t* p, size_t nparts, const uint64_t* parts, uint64_t* out) {
+int wl_rows_product_parts(wl_ctx* c, size_t n, const uint64_t* p, size_t nparts, const uint64_t* const* parts,
+                          uint64_t* out) {
     if (!c || nparts == 0 || nparts > (1u << 16) || n > (1ull << 32)) return WL_ERR_ARG;
     if (n == 0) return 0;
     if (!p || !parts || !out) return WL_ERR_ARG;
-    for (size_t i = 0; i < n; ++i)
-        if (p[i] < 5 || p[i] > WL_MAXP || !(p[i] & 1)) return WL_ERR_ARG;
-    for (size_t k = 0; k < nparts; ++k) {   // part by part, in memory order
-        const uint64_t* d = parts + k * 2 * n;
-        bool bad = false;
-        for (size_t i = 0; i < n; ++i) bad |= (d[2 * i] >= p[i]) | (d[2 * i + 1] >= p[i]);
-        if (bad) return WL_ERR_ARG;
-    }
+    for (size_t k = 0; k < nparts; ++k)
+        if (!parts[k]) return WL_ERR_ARG;
     cudaSetDevice(c->device);
-    const size_t pb = n * 8, xb = nparts * n * 16, ob = n * 16;
-    RC(ensure(c->prod, pb + xb + ob));
+    const size_t pb = n * 8, xb = n * 16, ob = n * 16;
+    RC(ensure(c->prod, pb + nparts * xb + ob + 16));
     uint64_t* dp = as<uint64_t>(c->prod);
     uint64_t* dx = dp + n;
     uint64_t* dout = dx + 2 * nparts * n;
+    uint32_t* dbad = (uint32_t*)(dout + 2 * n);
+    CK(cudaMemsetAsync(dbad, 0, 4, c->st));
     CK(cudaMemcpyAsync(dp, p, pb, cudaMemcpyHostToDevice, c->st));
-    CK(cudaMemcpyAsync(dx, parts, xb, cudaMemcpyHostToDevice, c->st));
-    launch_rows_product(dp, n, dx, (uint32_t)nparts, dout, c->st);
+    for (size_t k = 0; k < nparts; ++k)
+        CK(cudaMemcpyAsync(dx + 2 * k * n, parts[k], xb, cudaMemcpyHostToDevice, c->st));
+    launch_rows_product(dp, n, dx, (uint32_t)nparts, dout, WL_MAXP, dbad, c->st);
     CK(cudaGetLastError());
+    uint32_t bad = 0;
+    CK(cudaMemcpyAsync(&bad, dbad, 4, cudaMemcpyDeviceToHost, c->st));
+    CK(cudaStreamSynchronize(c->st));
+    if (bad) return WL_ERR_ARG;
     CK(cudaMemcpyAsync(out, dout, ob, cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
     return 0;
+}
+
+int wl_rows_product(wl_ctx* c, size_t n, const uint64_t* p, size_t nparts, const uint64_t* parts, uint64_t* out) {
+    if (!parts && n) return WL_ERR_ARG;
+    if (nparts > (1u << 16)) return WL_ERR_ARG;
+    std::vector<const uint64_t*> each(nparts);
+    for (size_t k = 0; k < nparts; ++k) each[k] = parts + k * 2 * n;
+    return wl_rows_product_parts(c, n, p, nparts, each.data(), out);
 }
 
 int wl_batch(wl_ctx* c, const wl_range* ranges, size_t n, uint64_t q_cap, wl_range_result* out,

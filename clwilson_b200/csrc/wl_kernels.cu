@@ -1288,7 +1288,9 @@ k_finish(const Bucket* __restrict__ buckets, const RowInfo* __restrict__ info, c
 // values s0 + p*s1 < p^2; their product is the running product over the union
 // of the pieces (the role of reduce.cl:11-44, which folds work-group partials
 // into a residue, one level up).  parts[k * 2n + 2i + {0, 1}] = digits of row
-// i's k-th partial; out[2i + {0, 1}] = digits of the product.
+// i's k-th partial; out[2i + {0, 1}] = digits of the product.  The inputs are
+// checked here, where every digit is read anyway: a modulus that is even, below
+// 5 or above p_max, or a digit that is not below its modulus, sets *bad.
 // ===========================================================================
 
 template <int L>
@@ -1321,10 +1323,19 @@ __device__ void rows_product_one(uint64_t p, const uint64_t* __restrict__ parts,
 
 __global__ void __launch_bounds__(128)
 k_rows_product(const uint64_t* __restrict__ ps, uint64_t n_rows, const uint64_t* __restrict__ parts, uint32_t nparts,
-               uint64_t* __restrict__ out) {
+               uint64_t* __restrict__ out, uint64_t p_max, uint32_t* __restrict__ bad) {
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n_rows) return;
     const uint64_t p = ps[i];
+    bool ok = p >= 5 && p <= p_max && (p & 1);
+    for (uint32_t k = 0; k < nparts; ++k) {
+        const uint64_t* d = parts + (uint64_t)k * 2 * n_rows + 2 * i;
+        ok &= d[0] < p && d[1] < p;
+    }
+    if (!ok) {
+        *bad = 1;
+        return;
+    }
     uint64_t d0, d1;
     if (p < (1ull << 31)) rows_product_one<2>(p, parts, n_rows, nparts, i, &d0, &d1);
     else if (p < (1ull << 47)) rows_product_one<3>(p, parts, n_rows, nparts, i, &d0, &d1);
@@ -2117,9 +2128,9 @@ void launch_finish(int L, const Bucket* buckets, const RowInfo* info, const RowM
     else k_finish<4><<<g, 128, 0, st>>>(buckets, info, mods, part, defs, K, ipart, row_begin, nrows, full, out, acc1, def1, acc2, def2, acc1 != nullptr);
 }
 void launch_rows_product(const uint64_t* ps, uint64_t n_rows, const uint64_t* parts, uint32_t nparts, uint64_t* out,
-                         cudaStream_t st) {
+                         uint64_t p_max, uint32_t* bad, cudaStream_t st) {
     if (!n_rows || !nparts) return;
-    k_rows_product<<<(unsigned)((n_rows + 127) / 128), 128, 0, st>>>(ps, n_rows, parts, nparts, out);
+    k_rows_product<<<(unsigned)((n_rows + 127) / 128), 128, 0, st>>>(ps, n_rows, parts, nparts, out, p_max, bad);
 }
 
 }  // namespace wl

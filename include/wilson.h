@@ -25,7 +25,7 @@
  *   wl_rows_from /        a search in pieces of columns with checkpoints (the
  *   wl_search_from        chunked main loop and resume, cl_wilson.cpp:1742-1776,
  *                         1856-1929)
- *   wl_rows_product       the fold of partial products into residues
+ *   wl_rows_product(_parts) the fold of partial products into residues
  *                         (reduce.cl:11-44) across the column pieces of GPUs
  *   wl_batch              many ranges in one device pass (no counterpart: the
  *                         reference runs one range per process)
@@ -180,6 +180,10 @@ int wl_search_from(wl_ctx *ctx, uint64_t pmin, uint64_t pmax, uint64_t q_lo, con
  * mod p[i]^2.  Computed on the GPU; WL_ERR_ARG for a bad p or digit. */
 int wl_rows_product(wl_ctx *ctx, size_t n, const uint64_t *p, size_t nparts, const uint64_t *parts,
                     uint64_t *out);
+
+/* As wl_rows_product, with each part's 2n digits in an array of its own. */
+int wl_rows_product_parts(wl_ctx *ctx, size_t n, const uint64_t *p, size_t nparts, const uint64_t *const *parts,
+                          uint64_t *out);
 
 /* Forget the resident column table; the next call sieves it again. */
 void wl_drop_columns(wl_ctx *ctx);
