@@ -358,38 +358,15 @@ __device__ __forceinline__ Res<L> mont_mul(const Res<L>& a, const Res<L>& b, con
     return r;
 }
 
-// Montgomery step with a 64-bit multiplier v < 2^63: x*v / 2^64 mod n.
-// Two rounds of the cell recurrence; x < 2n -> result < 2n.
+// Montgomery step with a 64-bit multiplier v < 2^63: x*v / 2^64 mod n, two limb
+// steps.  x < 2n: t stays below 3n in between and ends below x/2 + n < 2n.
 template <int L>
 __device__ __forceinline__ void cell64(Res<L>& x, uint64_t v, const uint32_t* n, uint32_t ninv) {
-    uint32_t t[L + 2];
+    uint32_t t[L];
 #pragma unroll
-    for (int i = 0; i < L + 2; ++i) t[i] = 0;
-    const uint32_t vw[2] = { (uint32_t)v, (uint32_t)(v >> 32) };
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        uint64_t c = 0;
-#pragma unroll
-        for (int j = 0; j < L; ++j) {
-            uint64_t s = (uint64_t)x.w[j] * vw[i] + t[j] + c;
-            t[j] = (uint32_t)s;
-            c = s >> 32;
-        }
-        uint64_t s = (uint64_t)t[L] + c;
-        t[L] = (uint32_t)s;
-        t[L + 1] = (uint32_t)(s >> 32);
-        uint32_t m = t[0] * ninv;
-        c = ((uint64_t)m * n[0] + t[0]) >> 32;
-#pragma unroll
-        for (int j = 1; j < L; ++j) {
-            uint64_t s2 = (uint64_t)m * n[j] + t[j] + c;
-            t[j - 1] = (uint32_t)s2;
-            c = s2 >> 32;
-        }
-        s = (uint64_t)t[L] + c;
-        t[L - 1] = (uint32_t)s;
-        t[L] = t[L + 1] + (uint32_t)(s >> 32);
-    }
+    for (int i = 0; i < L; ++i) t[i] = 0;
+    limb_step<L>(t, x, (uint32_t)v, n, ninv);
+    limb_step<L>(t, x, (uint32_t)(v >> 32), n, ninv);
 #pragma unroll
     for (int i = 0; i < L; ++i) x.w[i] = t[i];
 }
