@@ -60,6 +60,7 @@ sys.path.insert(0, ROOT)
 
 PLAIN_SMALL = (10**9, 10**6)
 OPS_PER_CELL = {2: 9, 3: 13, 4: 17}   # multiply-class PTX ops of one cell step (wl_arith.cuh)
+BF16_FALLBACK_TFLOPS = 1590.0
 HBM_FALLBACK_GBS = 6650.0             # copy bandwidth measured earlier on this kind of GPU
 
 
@@ -75,6 +76,19 @@ def hbm_peak():
     except Exception:
         pass
     return HBM_FALLBACK_GBS, "of fallback"
+
+
+def tensor_peak():
+    """(operations/s, source) of the 8-bit integer tensor roofline: nominally
+    twice the bf16 rate, which is measured."""
+    try:
+        with open(os.path.join(ROOT, "MEASURED_PEAKS.json")) as f:
+            v = json.load(f).get("bf16_tflops")
+        if v:
+            return 2e12 * float(v), "2 x bf16_tflops (of measured)"
+    except Exception:
+        pass
+    return 2e12 * BF16_FALLBACK_TFLOPS, "2 x bf16 (of fallback)"
 
 
 def work_cells(st, L):
@@ -765,6 +779,17 @@ def main():
             traffic = json.load(open(tpath)).get(args.workload)
         except Exception:
             traffic = None
+    # the tensor-core products' 8-bit operations over the sweep phase, which also
+    # holds their digit sort, group products and label folds
+    macs = sum(s.tensor_macs for s in stats)
+    peak_i8, i8_src = tensor_peak()
+    tensor_roofline = {
+        "bound": "tensor_i8", "achieved": 2.0 * macs / sweep_s / 1e12, "peak": peak_i8 / 1e12, "unit": "TOP/s",
+        "frac": 2.0 * macs / sweep_s / peak_i8, "traffic": None, "kernel": f"k_tensor_gemm<{L},*>",
+        "peak_source": i8_src, "macs_per_step": macs / args.steps,
+        "count": "8-bit multiply-accumulates of the products executed (128 groups x 256 row bytes x 512 bytes a "
+                 "tile, padding included), over the whole sweep phase",
+    }
     line = {
         "metric": "primes tested/s" if full else "128-bit mulmods/s (capped column sweep)",
         "value": (tested_all / tot_dev) if full else (cells_all / tot_dev),
@@ -779,7 +804,8 @@ def main():
                    "l2": "256 MiB buffer written between steps", "columns": "re-sieved every step",
                    "parallelism": f"rows sharded by range, dp{world}"},
         "mulmods_per_s": cells_all / tot_dev,
-        "roofline": {"bound": "imad", "achieved": achieved, "peak": peak_mad / 1e12, "unit": "TOP/s",
+        "roofline": tensor_roofline if macs else
+                    {"bound": "imad", "achieved": achieved, "peak": peak_mad / 1e12, "unit": "TOP/s",
                      "frac": achieved * 1e12 / peak_mad, "traffic": traffic,
                      "traffic_source": ("dram__bytes_read.sum + dram__bytes_write.sum of the step's sweep launches of "
                                         "this workload, one ncu capture (profiles/traffic.json)") if traffic else None,

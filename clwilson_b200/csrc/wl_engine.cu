@@ -505,6 +505,7 @@ static int run_ranges(wl_ctx* c, const wl_range* ranges, size_t nr, uint64_t qca
     c->h2d = c->d2h = 0;
     c->ms_sieve = 0;
     c->sieve_ints = c->sieve_bytes = 0;
+    c->tensor_macs = 0;
     c->ms_big = 0;
     for (size_t i = 0; i < nr; ++i) RC(wl_check_range(ranges[i].pmin, ranges[i].pmax));
 
@@ -1059,6 +1060,7 @@ static int run_ranges(wl_ctx* c, const wl_range* ranges, size_t nr, uint64_t qca
         st->dense_products = dwork[2];
         st->graph_nodes = cg.nodes;
         st->ms_graph_build = cg.ms_build;
+        st->tensor_macs = c->tensor_macs;
     }
     return 0;
 }
@@ -1201,7 +1203,8 @@ void wl_close(wl_ctx* c) {
                        &c->defs, &c->rowout, &c->prod, &c->windesc, &c->seglo, &c->work,
                        &c->tb.desc, &c->tb.counts, &c->tb.cursor, &c->tb.lab_seg, &c->tb.runs, &c->tb.segs, &c->tb.tables, &c->tb.list, &c->tb.w, &c->tb.consts, &c->tb.ones,
                        &c->tb.part, &c->tb.seg, &c->tb.win, &c->gprod, &c->gk };
-    for (DevBuf* b : bufs) if (b->p) cudaFree(b->p);
+    for (DevBuf* b : bufs) release(*b);
+    release(c->tb.block);
     for (auto& e : c->ev) if (e) cudaEventDestroy(e);
     if (c->fork) cudaEventDestroy(c->fork);
     if (c->join) cudaEventDestroy(c->join);

@@ -16,13 +16,16 @@
 struct DevBuf {
     void* p = nullptr;
     size_t cap = 0;
+    bool inner = false;    // lies in another buffer (TensorBufs::block): not freed by itself
 };
+inline void release(DevBuf& b) {
+    if (b.p && !b.inner) cudaFree(b.p);
+    b = DevBuf();
+}
 
 inline int ensure(DevBuf& b, size_t bytes) {
     if (bytes <= b.cap && b.p) return 0;
-    if (b.p) cudaFree(b.p);
-    b.p = nullptr;
-    b.cap = 0;
+    release(b);
     size_t nb = std::max<size_t>(bytes, 256);
     if (cudaMalloc(&b.p, nb) != cudaSuccess) {
         cudaGetLastError();
@@ -116,6 +119,7 @@ inline int limb_width(uint64_t pmax_incl) {
 
 // Workspace of the tensor-core column products (wl_tensor_host.cu).
 struct TensorBufs {
+    DevBuf block;          // one allocation that holds all of them while they are small
     DevBuf desc, counts, cursor, lab_seg, runs, segs, tables, list, w, consts, ones, part, seg, win;
 };
 
@@ -150,6 +154,7 @@ struct wl_ctx {
     uint64_t h2d = 0, d2h = 0;
     double ms_sieve = 0;
     uint64_t sieve_ints = 0, sieve_bytes = 0;
+    uint64_t tensor_macs = 0;   // of the current call
     DevBuf work;         // dense sweep work counters: column cells, window cells, products; then the
                          // tensor-core product's error word
     TensorBufs tb;

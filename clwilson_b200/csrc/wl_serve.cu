@@ -111,8 +111,9 @@ struct wl_server {
     uint64_t step_cells = 0;
     uint32_t shares = WL_SHARES_LEAST_WORK;
     DevBuf info, mods, acc, out, pbuckets, bdef, ipart;
-    DevBuf terr;                               // error word of the tensor-core products
+    uint32_t* terr = nullptr;                  // error word of the tensor-core products (behind bdef)
     size_t tbudget = 0;                        // workspace they may take (0: none, the sweeps run)
+    bool tbudget_known = false;                // asked for at the first admission
     // Two sets of a step's buffers: the scheduler plans and queues step k+1
     // into one set while step k still runs on the other, and completes step k
     // (its timing, the requests whose lift followed it) meanwhile.
@@ -209,6 +210,10 @@ static void serve_admit_batch(wl_server* s, const std::vector<SReq*>& cands, std
     wl_ctx* c = s->c;
     const size_t nc = cands.size();
     result.assign(nc, 1);
+    if (!s->tbudget_known) {
+        s->tbudget_known = true;
+        if (tensor_enabled()) s->tbudget = tensor_budget(c, 1e9, 1e6);   // what a large step would take
+    }
     cudaEventRecord(s->e0, c->st);
     // 1. test primes of the candidates that have none yet
     {
@@ -680,7 +685,7 @@ static int serve_step(wl_server* s) {
     if (!tensor.empty()) {
         // waits for the step before it; its own kernels then run beside the planning below
         const uint32_t before = c->launches;
-        RC(tensor_products(c, tensor, { as<RowMod>(s->mods), as<uint4>(s->acc), as<uint32_t>(s->terr) }, s->tbudget));
+        RC(tensor_products(c, tensor, { as<RowMod>(s->mods), as<uint4>(s->acc), s->terr }, s->tbudget));
         s->ws.launches += c->launches - before;
         sl.tensor = true;
     }
@@ -828,7 +833,7 @@ static void serve_complete(wl_server* s, wl_server::Slot& sl, int err = 0) {
     if (!err && cudaEventSynchronize(sl.e1) != cudaSuccess) err = WL_ERR_CUDA;
     if (!err && sl.tensor) {
         uint32_t ran_out = 0;
-        if (cudaMemcpyAsync(&ran_out, s->terr.p, 4, cudaMemcpyDeviceToHost, s->c->st3) != cudaSuccess ||
+        if (cudaMemcpyAsync(&ran_out, s->terr, 4, cudaMemcpyDeviceToHost, s->c->st3) != cudaSuccess ||
             cudaStreamSynchronize(s->c->st3) != cudaSuccess || ran_out)
             err = WL_ERR_CUDA;
     }
@@ -974,18 +979,17 @@ int wl_server_open(const wl_server_opts* opts, wl_server** out) {
     s->pool.reset(s->pool_cap);
     if (ensure(s->info, (size_t)s->pool_cap * sizeof(RowInfo)) || ensure(s->mods, (size_t)s->pool_cap * sizeof(RowMod)) ||
         ensure(s->acc, (size_t)s->pool_cap * 16) || ensure(s->out, (size_t)s->pool_cap * sizeof(RowOut)) ||
-        ensure(s->pbuckets, s->bucket_cap * sizeof(Bucket)) || ensure(s->bdef, s->bucket_cap * sizeof(Deficit)) ||
-        ensure(s->terr, 16) || cudaMemset(s->terr.p, 0, 16) != cudaSuccess || cudaEventCreate(&s->e0) != cudaSuccess || cudaEventCreate(&s->e1) != cudaSuccess ||
+        ensure(s->pbuckets, s->bucket_cap * sizeof(Bucket)) || ensure(s->bdef, s->bucket_cap * sizeof(Deficit) + 16) ||
+        cudaEventCreate(&s->e0) != cudaSuccess || cudaEventCreate(&s->e1) != cudaSuccess ||
         cudaEventCreate(&s->slot[0].e0) != cudaSuccess || cudaEventCreate(&s->slot[0].e1) != cudaSuccess ||
         cudaEventCreate(&s->slot[1].e0) != cudaSuccess || cudaEventCreate(&s->slot[1].e1) != cudaSuccess) {
         cudaGetLastError();
-        DevBuf* bufs[] = { &s->info, &s->mods, &s->acc, &s->out, &s->pbuckets, &s->bdef, &s->terr };
+        DevBuf* bufs[] = { &s->info, &s->mods, &s->acc, &s->out, &s->pbuckets, &s->bdef };
         for (DevBuf* b : bufs) if (b->p) cudaFree(b->p);
         wl_close(s->c);
         delete s;
         return WL_ERR_NOMEM;
     }
-    if (tensor_enabled()) s->tbudget = tensor_budget(s->c, 1e9, 1e6);   // what a large call would take
     // the step buffers' pool, which keeps what is freed into it; each set of
     // step buffers starts at the size a step of the default budget takes
     // (about two rows of split products per thread of the sweep, a split
@@ -1009,6 +1013,8 @@ int wl_server_open(const wl_server_opts* opts, wl_server** out) {
         wl_server_close(s);                              // no worker yet: frees what there is
         return WL_ERR_NOMEM;
     }
+    s->terr = (uint32_t*)(as<Deficit>(s->bdef) + s->bucket_cap);
+    cudaMemset(s->terr, 0, 16);
     cudaMemset(s->pbuckets.p, 0, s->bucket_cap * sizeof(Bucket));
     cudaMemset(s->info.p, 0, (size_t)s->pool_cap * sizeof(RowInfo));   // bucket 0 for rows never admitted
     s->worker = std::thread(serve_loop, s);
@@ -1138,7 +1144,7 @@ void wl_server_close(wl_server* s) {
     if (s->worker.joinable()) s->worker.join();
     cudaSetDevice(s->c->device);
     cudaStreamSynchronize(s->c->st);
-    DevBuf* bufs[] = { &s->info, &s->mods, &s->acc, &s->out, &s->pbuckets, &s->bdef, &s->ipart, &s->terr };
+    DevBuf* bufs[] = { &s->info, &s->mods, &s->acc, &s->out, &s->pbuckets, &s->bdef, &s->ipart };
     for (DevBuf* b : bufs) if (b->p) cudaFree(b->p);
     for (auto& sl : s->slot) {
         DevBuf* sb[] = { &sl.sbuckets, &sl.items, &sl.part, &sl.defs, &sl.bbitmap, &sl.bsegcount, &sl.boffs,

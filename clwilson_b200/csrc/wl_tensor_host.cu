@@ -64,6 +64,35 @@ uint32_t row_tiles_of(uint32_t nrows, int L) { return (nrows + tn_rows(L) - 1) /
 
 // Shares of the workspace: group lists and products together, lane-run
 // products, row constants.  Tasks are cut so that a chunk keeps within them.
+// A buffer that must grow grows by half, so that calls and steps of slowly rising
+// size do not free and allocate each time.
+int grow(DevBuf& b, size_t bytes) { return bytes <= b.cap && b.p ? 0 : ensure(b, std::max(bytes, b.cap + b.cap / 2)); }
+
+// The workspace of a small call in one allocation: a dozen of them would be most
+// of a small search's first call (each some 0.1 ms).
+int first_block(TensorBufs& tb) {
+    if (tb.block.p) return 0;
+    struct Part { DevBuf* b; size_t bytes; };
+    const Part parts[] = { { &tb.w, 4u << 20 },       { &tb.consts, 2u << 20 },   { &tb.list, 1u << 20 },
+                           { &tb.part, 1u << 20 },    { &tb.seg, 256u << 10 },    { &tb.win, 256u << 10 },
+                           { &tb.runs, 128u << 10 },  { &tb.counts, 64u << 10 },  { &tb.cursor, 64u << 10 },
+                           { &tb.lab_seg, 64u << 10 }, { &tb.segs, 64u << 10 },   { &tb.tables, 64u << 10 },
+                           { &tb.ones, 64u << 10 },   { &tb.desc, 16u << 10 } };
+    size_t total = 0;
+    for (const Part& p : parts) total += p.bytes;
+    RC(ensure(tb.block, total));
+    uint8_t* at = as<uint8_t>(tb.block);
+    for (const Part& p : parts) {
+        if (!p.b->p) {
+            p.b->p = at;
+            p.b->cap = p.bytes;
+            p.b->inner = true;
+        }
+        at += p.bytes;
+    }
+    return 0;
+}
+
 struct Limits {
     double entries, part, consts;
 };
@@ -144,6 +173,7 @@ uint32_t Products::slab_rows(const TensorTask& t, const TensorSize& z) const {
 // Counts the digits of tasks [t0, t1) (one launch, one wait for their sizes), then runs them in chunks.
 int Products::wave(size_t t0, size_t t1) {
     cudaStream_t st = c->st;
+    RC(first_block(tb));
     const uint32_t nt = (uint32_t)(t1 - t0);
     desc.assign(nt, TensorDesc());
     size.assign(nt, TensorSize());
@@ -164,10 +194,10 @@ int Products::wave(size_t t0, size_t t1) {
         nblk += (d.c1 - d.c0 + TN_COLS_PER_BLOCK - 1) / TN_COLS_PER_BLOCK;
     }
     const size_t size_at = ((size_t)nt * sizeof(TensorDesc) + 255) & ~size_t(255);
-    RC(ensure(tb.desc, size_at + nt * sizeof(TensorSize)));
-    RC(ensure(tb.counts, (size_t)nlab * 4 + 16));
-    RC(ensure(tb.cursor, (size_t)nlab * 4 + 16));
-    RC(ensure(tb.lab_seg, (size_t)(nlab + nt) * 4 + 16));
+    RC(grow(tb.desc, size_at + nt * sizeof(TensorSize)));
+    RC(grow(tb.counts, (size_t)nlab * 4 + 16));
+    RC(grow(tb.cursor, (size_t)nlab * 4 + 16));
+    RC(grow(tb.lab_seg, (size_t)(nlab + nt) * 4 + 16));
     TensorSize* dsize = (TensorSize*)(as<uint8_t>(tb.desc) + size_at);
     CK(cudaMemcpyAsync(tb.desc.p, desc.data(), nt * sizeof(TensorDesc), cudaMemcpyHostToDevice, st));
     CK(cudaMemsetAsync(tb.counts.p, 0, (size_t)nlab * 4, st));
@@ -211,12 +241,12 @@ int Products::wave(size_t t0, size_t t1) {
         segs = std::max(segs, ns);
         i = j;
     }
-    RC(ensure(tb.list, list * 4 + 16));
-    RC(ensure(tb.w, w + 16));
-    RC(ensure(tb.part, part + 16));
-    RC(ensure(tb.consts, consts + 16));
-    RC(ensure(tb.runs, runs * sizeof(LaneRun) + 16));
-    RC(ensure(tb.segs, segs * sizeof(FoldSeg) + 16));
+    RC(grow(tb.list, list * 4 + 16));
+    RC(grow(tb.w, w + 16));
+    RC(grow(tb.part, part + 16));
+    RC(grow(tb.consts, consts + 16));
+    RC(grow(tb.runs, runs * sizeof(LaneRun) + 16));
+    RC(grow(tb.segs, segs * sizeof(FoldSeg) + 16));
     for (auto& x : chunks) RC(chunk(tasks.data() + t0, x.first, x.second));
     return 0;
 }
@@ -279,6 +309,7 @@ int Products::chunk(const TensorTask* ts, size_t i0, size_t i1) {
             win += (uint64_t)((d.nwin << d.w) / TN_DIGITS) * d.rows_pad;
             units += (uint64_t)group_tiles(size[i0 + i]) * tiles;
         }
+        c->tensor_macs += units * TN_M * TN_N * TN_K;
         // items of 32 to 256 group tiles, about eight per SM where the work allows:
         // shorter ones would show the 128 KB of constants that each brings in
         const uint64_t per_item = std::min<uint64_t>(256, std::max<uint64_t>(32, units / ((uint64_t)c->sms * 8)));
@@ -294,11 +325,11 @@ int Products::chunk(const TensorTask* ts, size_t i0, size_t i1) {
         }
         Tables tab;
         const size_t o_desc = tab.add(dc), o_sec = tab.add(secs), o_item = tab.add(items);
-        RC(ensure(tb.ones, (size_t)ntile * rt * 16 + 16));
-        RC(ensure(tb.tables, tab.bytes.size()));
-        RC(ensure(tb.seg, seg * esz + 16));
-        RC(ensure(tb.win, win * esz + 16));
-        RC(ensure(tb.part, part * esz + 16));
+        RC(grow(tb.ones, (size_t)ntile * rt * 16 + 16));
+        RC(grow(tb.tables, tab.bytes.size()));
+        RC(grow(tb.seg, seg * esz + 16));
+        RC(grow(tb.win, win * esz + 16));
+        RC(grow(tb.part, part * esz + 16));
         CK(cudaMemcpyAsync(tb.tables.p, tab.bytes.data(), tab.bytes.size(), cudaMemcpyHostToDevice, st));
         c->h2d += tab.bytes.size();
         uint8_t* base = as<uint8_t>(tb.tables);
@@ -385,6 +416,7 @@ int tensor_products(wl_ctx* c, std::vector<TensorTask> tasks, const TensorTarget
 int tensor_tails(wl_ctx* c, const std::vector<TensorTail>& tails, const std::vector<RowInfo>& ri, const TensorTarget& to) {
     cudaStream_t st = c->st;
     TensorBufs& tb = c->tb;
+    RC(first_block(tb));
     for (size_t i0 = 0; i0 < tails.size();) {
         const int L = (int)tails[i0].L;
         const uint32_t rt = tn_rows(L);
@@ -429,11 +461,11 @@ int tensor_tails(wl_ctx* c, const std::vector<TensorTail>& tails, const std::vec
                          [](const TensorItem& a, const TensorItem& b) { return a.ncb > b.ncb; });
         Tables tab;
         const size_t o_desc = tab.add(dc), o_sec = tab.add(secs), o_item = tab.add(items);
-        RC(ensure(tb.tables, tab.bytes.size()));
-        RC(ensure(tb.consts, (size_t)ntile * TN_N * TN_K + 16));
-        RC(ensure(tb.ones, (size_t)ntile * rt * 16 + 16));
-        RC(ensure(tb.part, part * (L == 2 ? 8 : 16) + 16));
-        RC(ensure(tb.w, (size_t)nmt * TN_M * TN_K + 16));
+        RC(grow(tb.tables, tab.bytes.size()));
+        RC(grow(tb.consts, (size_t)ntile * TN_N * TN_K + 16));
+        RC(grow(tb.ones, (size_t)ntile * rt * 16 + 16));
+        RC(grow(tb.part, part * (L == 2 ? 8 : 16) + 16));
+        RC(grow(tb.w, (size_t)nmt * TN_M * TN_K + 16));
         CK(cudaMemcpyAsync(tb.tables.p, tab.bytes.data(), tab.bytes.size(), cudaMemcpyHostToDevice, st));
         c->h2d += tab.bytes.size();
         uint8_t* base = as<uint8_t>(tb.tables);
@@ -451,6 +483,7 @@ int tensor_tails(wl_ctx* c, const std::vector<TensorTail>& tails, const std::vec
                                 to.acc, st);
         CK(cudaGetLastError());
         c->launches += 4;
+        for (const TensorItem& it : items) c->tensor_macs += (uint64_t)it.ncb * TN_M * TN_N * TN_K;
         i0 = i1;
     }
     return 0;

@@ -125,6 +125,8 @@ typedef struct {
     uint64_t graph_nodes;       /* nodes of the CUDA graph that carried the call's sweep, merges,
                                    tail and lift (wl_batch); 0 when they were launched one by one */
     double ms_graph_build;      /* host time to end that graph's capture and instantiate it */
+    uint64_t tensor_macs;       /* 8-bit multiply-accumulates of the tensor-core products (0: the sweeps
+                                   took every bucket) */
 } wl_stats;
 
 /* Open a context on CUDA device `device`. */
