@@ -1647,11 +1647,23 @@ k_sweep_bits(const Bucket* __restrict__ buckets, const SweepItem* __restrict__ i
     u128 def = 0;
     uint64_t e_cur = 0, thr = 0, cells = 0;
     bool started = false;
-    for (uint64_t w = w0; w < w1; ++w) {
-        uint32_t word = __ldg(bitmap + w);
-        const uint64_t qb = lo + 64 * w + 1;
-        while (word) {
-            const int b = __ffs(word) - 1;
+    // Four words at a time: the lanes of a warp work on several splits, and the
+    // warp stays with a block of words until the fullest of them is done (64
+    // integers hold 2.8 primes on average but 5.5 in the fullest of seven splits,
+    // 256 hold 11.4 and 15.7; 20 rows past 2^32: 7.88 ms, 8.07 with single words).
+    // Regions start at a multiple of four words and are whole segments long.
+    for (uint64_t w = w0 & ~3ull; w < w1; w += 4) {
+        const uint4 v = __ldg(reinterpret_cast<const uint4*>(bitmap + w));
+        uint64_t word = (w >= w0 ? v.x : 0u) | (uint64_t)(w + 1 >= w0 && w + 1 < w1 ? v.y : 0u) << 32;
+        uint64_t next = (w + 2 >= w0 && w + 2 < w1 ? v.z : 0u) | (uint64_t)(w + 3 < w1 ? v.w : 0u) << 32;
+        uint64_t qb = lo + 64 * w + 1;
+        while (word | next) {
+            if (word == 0) {
+                word = next;
+                next = 0;
+                qb += 128;
+            }
+            const int b = __ffsll((long long)word) - 1;
             word &= word - 1;
             const uint64_t q = qb + 2ull * b;
             if (q > key) { w = w1; break; }
