@@ -1200,11 +1200,9 @@ void wl_close(wl_ctx* c) {
                        &c->buckets, &c->rowinfo, &c->rowmod, &c->items, &c->part, &c->ipart, &c->dsplit,
                        &c->bbitmap, &c->bsegcount, &c->boffsets, &c->boffs, &c->wcols, &c->wbuckets, &c->witems,
                        &c->wpart, &c->wdefs, &c->bacc, &c->bdef, &c->wkeys, &c->wcounts, &c->uacc, &c->udef,
-                       &c->defs, &c->rowout, &c->prod, &c->windesc, &c->seglo, &c->work,
-                       &c->tb.desc, &c->tb.counts, &c->tb.cursor, &c->tb.lab_seg, &c->tb.runs, &c->tb.segs, &c->tb.tables, &c->tb.list, &c->tb.w, &c->tb.consts, &c->tb.ones,
-                       &c->tb.part, &c->tb.seg, &c->tb.win, &c->gprod, &c->gk };
+                       &c->defs, &c->rowout, &c->prod, &c->windesc, &c->seglo, &c->work, &c->gprod, &c->gk };
     for (DevBuf* b : bufs) release(*b);
-    release(c->tb.block);
+    tensor_release(c);
     for (auto& e : c->ev) if (e) cudaEventDestroy(e);
     if (c->fork) cudaEventDestroy(c->fork);
     if (c->join) cudaEventDestroy(c->join);

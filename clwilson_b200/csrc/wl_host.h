@@ -119,6 +119,8 @@ inline int limb_width(uint64_t pmax_incl) {
 
 // Workspace of the tensor-core column products (wl_tensor_host.cu).
 struct TensorBufs {
+    cudaMemPool_t pool = nullptr;   // serving: grow from this pool, in the order of `st` (ensure_step's reason)
+    cudaStream_t st = nullptr;
     DevBuf block;          // one allocation that holds all of them while they are small
     DevBuf desc, counts, cursor, lab_seg, runs, segs, tables, list, w, consts, ones, part, seg, win;
 };
@@ -182,6 +184,8 @@ struct RangeState {
 // device); with allow_empty a range without primes is not an error.
 int gen_test_primes(wl_ctx* c, const wl_range* ranges, size_t nr, std::vector<RangeState>& rs,
                     std::vector<uint64_t>& tps, bool allow_empty = false);
+// Frees the tensor-core products' workspace.
+void tensor_release(wl_ctx* c);
 // WL_TENSOR=0 in the environment turns the tensor-core products off, for comparisons.
 inline bool tensor_enabled() {
     static const bool off = getenv("WL_TENSOR") && atoi(getenv("WL_TENSOR")) == 0;

@@ -1003,6 +1003,10 @@ int wl_server_open(const wl_server_opts* opts, wl_server** out) {
     const uint64_t keep_all = ~0ull;
     bool ok = cudaMemPoolCreate(&s->mpool, &pp) == cudaSuccess &&
               cudaMemPoolSetAttribute(s->mpool, cudaMemPoolAttrReleaseThreshold, (void*)&keep_all) == cudaSuccess;
+    if (ok) {
+        s->c->tb.pool = s->mpool;
+        s->c->tb.st = s->c->st;
+    }
     const size_t threads = (size_t)s->c->sms * 2048 * 4;
     for (auto& sl : s->slot)
         ok = ok && !ensure_step(s, sl.sbuckets, (size_t)s->bucket_cap * sizeof(Bucket)) &&
@@ -1153,6 +1157,8 @@ void wl_server_close(wl_server* s) {
         if (sl.e0) cudaEventDestroy(sl.e0);
         if (sl.e1) cudaEventDestroy(sl.e1);
     }
+    tensor_release(s->c);                       // its buffers come from the pool too
+    s->c->tb.pool = nullptr;
     cudaStreamSynchronize(s->c->st);
     if (s->mpool) cudaMemPoolDestroy(s->mpool);
     if (s->e0) cudaEventDestroy(s->e0);

@@ -66,7 +66,22 @@ uint32_t row_tiles_of(uint32_t nrows, int L) { return (nrows + tn_rows(L) - 1) /
 // products, row constants.  Tasks are cut so that a chunk keeps within them.
 // A buffer that must grow grows by half, so that calls and steps of slowly rising
 // size do not free and allocate each time.
-int grow(DevBuf& b, size_t bytes) { return bytes <= b.cap && b.p ? 0 : ensure(b, std::max(bytes, b.cap + b.cap / 2)); }
+int grow(TensorBufs& tb, DevBuf& b, size_t bytes) {
+    if (bytes <= b.cap && b.p) return 0;
+    const size_t want = std::max(bytes, b.cap + b.cap / 2);
+    if (!tb.pool) return ensure(b, want);
+    if (b.p && !b.inner) cudaFreeAsync(b.p, tb.st);
+    b = DevBuf();
+    for (size_t n : { want, bytes }) {
+        if (cudaMallocFromPoolAsync(&b.p, n, tb.pool, tb.st) == cudaSuccess) {
+            b.cap = n;
+            return 0;
+        }
+        cudaGetLastError();
+        b.p = nullptr;
+    }
+    return WL_ERR_NOMEM;
+}
 
 // The workspace of a small call in one allocation: a dozen of them would be most
 // of a small search's first call (each some 0.1 ms).
@@ -194,10 +209,10 @@ int Products::wave(size_t t0, size_t t1) {
         nblk += (d.c1 - d.c0 + TN_COLS_PER_BLOCK - 1) / TN_COLS_PER_BLOCK;
     }
     const size_t size_at = ((size_t)nt * sizeof(TensorDesc) + 255) & ~size_t(255);
-    RC(grow(tb.desc, size_at + nt * sizeof(TensorSize)));
-    RC(grow(tb.counts, (size_t)nlab * 4 + 16));
-    RC(grow(tb.cursor, (size_t)nlab * 4 + 16));
-    RC(grow(tb.lab_seg, (size_t)(nlab + nt) * 4 + 16));
+    RC(grow(tb, tb.desc, size_at + nt * sizeof(TensorSize)));
+    RC(grow(tb, tb.counts, (size_t)nlab * 4 + 16));
+    RC(grow(tb, tb.cursor, (size_t)nlab * 4 + 16));
+    RC(grow(tb, tb.lab_seg, (size_t)(nlab + nt) * 4 + 16));
     TensorSize* dsize = (TensorSize*)(as<uint8_t>(tb.desc) + size_at);
     CK(cudaMemcpyAsync(tb.desc.p, desc.data(), nt * sizeof(TensorDesc), cudaMemcpyHostToDevice, st));
     CK(cudaMemsetAsync(tb.counts.p, 0, (size_t)nlab * 4, st));
@@ -241,12 +256,12 @@ int Products::wave(size_t t0, size_t t1) {
         segs = std::max(segs, ns);
         i = j;
     }
-    RC(grow(tb.list, list * 4 + 16));
-    RC(grow(tb.w, w + 16));
-    RC(grow(tb.part, part + 16));
-    RC(grow(tb.consts, consts + 16));
-    RC(grow(tb.runs, runs * sizeof(LaneRun) + 16));
-    RC(grow(tb.segs, segs * sizeof(FoldSeg) + 16));
+    RC(grow(tb, tb.list, list * 4 + 16));
+    RC(grow(tb, tb.w, w + 16));
+    RC(grow(tb, tb.part, part + 16));
+    RC(grow(tb, tb.consts, consts + 16));
+    RC(grow(tb, tb.runs, runs * sizeof(LaneRun) + 16));
+    RC(grow(tb, tb.segs, segs * sizeof(FoldSeg) + 16));
     for (auto& x : chunks) RC(chunk(tasks.data() + t0, x.first, x.second));
     return 0;
 }
@@ -325,11 +340,11 @@ int Products::chunk(const TensorTask* ts, size_t i0, size_t i1) {
         }
         Tables tab;
         const size_t o_desc = tab.add(dc), o_sec = tab.add(secs), o_item = tab.add(items);
-        RC(grow(tb.ones, (size_t)ntile * rt * 16 + 16));
-        RC(grow(tb.tables, tab.bytes.size()));
-        RC(grow(tb.seg, seg * esz + 16));
-        RC(grow(tb.win, win * esz + 16));
-        RC(grow(tb.part, part * esz + 16));
+        RC(grow(tb, tb.ones, (size_t)ntile * rt * 16 + 16));
+        RC(grow(tb, tb.tables, tab.bytes.size()));
+        RC(grow(tb, tb.seg, seg * esz + 16));
+        RC(grow(tb, tb.win, win * esz + 16));
+        RC(grow(tb, tb.part, part * esz + 16));
         CK(cudaMemcpyAsync(tb.tables.p, tab.bytes.data(), tab.bytes.size(), cudaMemcpyHostToDevice, st));
         c->h2d += tab.bytes.size();
         uint8_t* base = as<uint8_t>(tb.tables);
@@ -361,6 +376,21 @@ int Products::chunk(const TensorTask* ts, size_t i0, size_t i1) {
 }
 
 }  // namespace
+
+void tensor_release(wl_ctx* c) {
+    TensorBufs& tb = c->tb;
+    DevBuf* all[] = { &tb.w, &tb.consts, &tb.list, &tb.part, &tb.seg, &tb.win, &tb.runs, &tb.counts, &tb.cursor,
+                      &tb.lab_seg, &tb.segs, &tb.tables, &tb.ones, &tb.desc };
+    for (DevBuf* b : all) {
+        if (b->p && !b->inner && tb.pool) {
+            cudaFreeAsync(b->p, tb.st);
+            *b = DevBuf();
+        } else {
+            release(*b);
+        }
+    }
+    release(tb.block);
+}
 
 // The least free memory the tensor-core path takes on, and the most workspace it plans for.
 static constexpr size_t TENSOR_MIN_BUDGET = 1ull << 30, TENSOR_MAX_BUDGET = 2ull << 30;
@@ -461,11 +491,11 @@ int tensor_tails(wl_ctx* c, const std::vector<TensorTail>& tails, const std::vec
                          [](const TensorItem& a, const TensorItem& b) { return a.ncb > b.ncb; });
         Tables tab;
         const size_t o_desc = tab.add(dc), o_sec = tab.add(secs), o_item = tab.add(items);
-        RC(grow(tb.tables, tab.bytes.size()));
-        RC(grow(tb.consts, (size_t)ntile * TN_N * TN_K + 16));
-        RC(grow(tb.ones, (size_t)ntile * rt * 16 + 16));
-        RC(grow(tb.part, part * (L == 2 ? 8 : 16) + 16));
-        RC(grow(tb.w, (size_t)nmt * TN_M * TN_K + 16));
+        RC(grow(tb, tb.tables, tab.bytes.size()));
+        RC(grow(tb, tb.consts, (size_t)ntile * TN_N * TN_K + 16));
+        RC(grow(tb, tb.ones, (size_t)ntile * rt * 16 + 16));
+        RC(grow(tb, tb.part, part * (L == 2 ? 8 : 16) + 16));
+        RC(grow(tb, tb.w, (size_t)nmt * TN_M * TN_K + 16));
         CK(cudaMemcpyAsync(tb.tables.p, tab.bytes.data(), tab.bytes.size(), cudaMemcpyHostToDevice, st));
         c->h2d += tab.bytes.size();
         uint8_t* base = as<uint8_t>(tb.tables);
