@@ -234,6 +234,9 @@ int Products::wave(size_t t0, size_t t1) {
         for (; j < nt && tasks[t0 + j].L == tasks[t0 + i].L; ++j) {
             const TensorTask& t = tasks[t0 + j];
             const TensorSize& z = size[j];
+            // two pieces of one bucket multiply into the same rows: never in one chunk
+            // (pieces are neighbours; their entries may fall short of what cut them)
+            if (j > i && t.row_begin == tasks[t0 + j - 1].row_begin) break;
             const uint32_t rows = std::min(t.nrows, slab_rows(t, z)), tiles = row_tiles_of(rows, t.L);
             const double pe = (double)z.slots * tiles * tn_rows(t.L) * (t.L == 2 ? 8 : 16);
             const double ke = (double)tiles * TN_N * TN_K;

@@ -86,3 +86,17 @@ def test_batch_equals_single_ranges(engine):
     for (a, b), r in zip(ranges, per):
         one = engine.search(a, b, q_cap=1 << 21)
         assert r["checksum"] == one.checksum and r["tested"] == one.stats.tested
+
+
+def test_pieces_of_one_bucket(engine):
+    # The class of T = p/2 has 1.7e7 columns, planned at two list entries each and so
+    # cut in two pieces; exponents are below 256 from q = 1.6e8 on, so that the pieces
+    # together hold fewer entries than one chunk takes.  They share their rows.
+    lo, hi, qcap = 8 * 10**10, 8 * 10**10 + 20000, 320 * 10**6
+    rows, st = engine.rows(lo, hi, q_cap=qcap)
+    assert st.dense_column_cells == 0 and st.tensor_macs > 0
+    t = [int(i) for i in range(3) if st.targets[i] > lo // 3]
+    hit = np.nonzero(rows["type"] == t[0])[0] if t else np.arange(len(rows))
+    sel = hit[np.linspace(0, len(hit) - 1, 8).astype(int)].astype(np.uint32)
+    want, _ = oracle.search(lo, hi, qcap, rows=sel)
+    _same(rows, want, sel)
