@@ -435,7 +435,10 @@ class Engine:
             if x.dtype.names:
                 if not np.array_equal(x["p"], p):
                     raise ValueError("rows_product: the parts hold different primes")
-                digits.append(np.stack([x["s0"], x["s1"]], axis=1))
+                d = np.empty((n, 2), dtype=np.uint64)  # the fields of any integer type, as the library reads them
+                d[:, 0] = x["s0"]
+                d[:, 1] = x["s1"]
+                digits.append(d)
             else:
                 if x.shape != (n, 2):
                     raise ValueError("rows_product: a digit part must have shape (%d, 2)" % n)
