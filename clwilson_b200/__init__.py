@@ -127,7 +127,7 @@ assert ROW_DTYPE.itemsize == ctypes.sizeof(_Row)
 # exported symbols of include/wilson.h
 SYMBOLS = ("wl_open", "wl_close", "wl_strerror", "wl_stream", "wl_check_range", "wl_search", "wl_rows",
            "wl_batch", "wl_rows_from", "wl_search_from", "wl_rows_product", "wl_rows_product_parts",
-           "wl_drop_columns", "wl_parse_uint64",
+           "wl_drop_columns", "wl_set_wait_limit", "wl_parse_uint64",
            "wl_probe",
            "wl_column_product_noalloc", "wl_get_tuning", "wl_set_tuning", "wl_autotune",
            "wl_server_open", "wl_server_submit", "wl_server_poll", "wl_server_wait", "wl_server_results",
@@ -177,6 +177,8 @@ def load_library(path: str = LIB_PATH):
     L.wl_parse_uint64.restype = ctypes.c_int
     L.wl_drop_columns.argtypes = [vp]
     L.wl_drop_columns.restype = None
+    L.wl_set_wait_limit.argtypes = [vp, u64]
+    L.wl_set_wait_limit.restype = ctypes.c_int
     L.wl_probe.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.POINTER(ctypes.c_double)]
     L.wl_probe.restype = ctypes.c_int
     L.wl_column_product_noalloc.argtypes = [vp, ctypes.c_uint32, u64, u64, vp, ctypes.c_uint32, vp, vp]
@@ -322,6 +324,12 @@ class Engine:
 
     def drop_columns(self) -> None:
         self._L.wl_drop_columns(self._ctx)
+
+    def set_wait_limit(self, ns: int) -> None:
+        """Limit of a wait inside the tensor-core products' kernels (wl_set_wait_limit)."""
+        rc = self._L.wl_set_wait_limit(self._ctx, ns)
+        if rc:
+            raise WilsonError(rc, "wl_set_wait_limit")
 
     @property
     def tuning(self) -> dict:

@@ -1327,6 +1327,12 @@ int wl_batch(wl_ctx* c, const wl_range* ranges, size_t n, uint64_t q_cap, wl_ran
     return summarize(ro, n, q_cap == 0, out, results, cap, nresults, stats);
 }
 
+int wl_set_wait_limit(wl_ctx* c, uint64_t ns) {
+    if (!c) return WL_ERR_ARG;
+    c->wait_ns = ns;
+    return 0;
+}
+
 int wl_get_tuning(wl_ctx* c, wl_tuning* out) {
     if (!c || !out) return WL_ERR_ARG;
     *out = c->tune;

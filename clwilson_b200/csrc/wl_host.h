@@ -2,6 +2,7 @@
 // serving session (wl_serve.cu): device buffers, error macros, the context.
 #pragma once
 #include <algorithm>
+#include <atomic>
 #include <cstdio>
 #include <cstdlib>
 #include <vector>
@@ -125,6 +126,8 @@ struct TensorBufs {
     DevBuf desc, counts, cursor, lab_seg, runs, segs, tables, list, w, consts, ones, part, seg, win;
 };
 
+constexpr uint64_t WAIT_NS = 4000000000ull;
+
 struct wl_ctx {
     int device = 0;
     int sms = 148;
@@ -157,6 +160,7 @@ struct wl_ctx {
     double ms_sieve = 0;
     uint64_t sieve_ints = 0, sieve_bytes = 0;
     uint64_t tensor_macs = 0;   // of the current call
+    std::atomic<uint64_t> wait_ns{ WAIT_NS };   // limit of a wait inside the tensor-core products' kernels
     DevBuf work;         // dense sweep work counters: column cells, window cells, products; then the
                          // tensor-core product's error word
     TensorBufs tb;

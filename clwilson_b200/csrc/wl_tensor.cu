@@ -606,9 +606,10 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
         : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok != 0;
 }
-// Waits for the phase, for about four seconds at most (a step of a wait is
-// bounded by the hardware); false when the limit was reached.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
+// Waits for the phase, for about limit_ns at most (a step of a wait is bounded
+// by the hardware); false when the limit was reached, with a limit of 0 at once.
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint64_t limit_ns) {
+    if (limit_ns == 0) return false;
     if (mbar_try(bar, parity)) return true;
     uint64_t t0, t;
     asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
@@ -616,7 +617,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
         if (mbar_try(bar, parity)) return true;
         if ((k & 255u) == 255u) {
             asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-            if (t - t0 > 4000000000ull) break;
+            if (t - t0 > limit_ns) break;
         }
     }
     return false;
@@ -626,6 +627,9 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
                  "l"(src), "r"(bytes), "r"(bar)
                  : "memory");
 }
+// What a CTA has in flight when one of its waits has run out ends before its
+// shared and tensor memory go: these waits have a limit of their own.
+constexpr uint64_t TG_DRAIN_NS = 4000000000ull;
 // Shared-memory descriptor of a K-major operand block: rows of 128 bytes, 128-byte
 // swizzle, groups of eight rows 1,024 bytes apart.
 __device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
@@ -745,14 +749,14 @@ k_tensor_gemm(const TensorDesc* __restrict__ desc, const TensorSec* __restrict__
               const TensorItem* __restrict__ items, const LaneRun* __restrict__ lr, const RowInfo* __restrict__ info,
               const RowMod* __restrict__ mods,
               const uint8_t* __restrict__ w, const uint8_t* __restrict__ consts, const uint4* __restrict__ ones,
-              typename PartOf<L>::T* __restrict__ part, uint32_t* __restrict__ err) {
+              typename PartOf<L>::T* __restrict__ part, uint32_t* __restrict__ err, uint64_t wait_ns) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_addr(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
     const uint32_t sB = base, sA = base + TN_KB * TG_B_BYTES;
     const uint32_t bars = sA + TG_STAGES * TG_A_BYTES;
     const uint32_t bFull = bars, bEmpty = bars + 8 * TG_STAGES, bConst = bEmpty + 8 * TG_STAGES;
-    const uint32_t bAccFull = bConst + 8, bAccEmpty = bAccFull + 16, sTmem = bAccEmpty + 16;
+    const uint32_t bAccFull = bConst + 8, bAccEmpty = bAccFull + 16, bLast = bAccEmpty + 16, sTmem = bLast + 8;
     const uint32_t wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const TensorItem it = items[blockIdx.x];
     const TensorSec sec = secs[it.sec];
@@ -761,6 +765,7 @@ k_tensor_gemm(const TensorDesc* __restrict__ desc, const TensorSec* __restrict__
     if (threadIdx.x == 0) {
         for (uint32_t s = 0; s < TG_STAGES; ++s) { mbar_init(bFull + 8 * s, 1); mbar_init(bEmpty + 8 * s, 1); }
         mbar_init(bConst, 1);
+        mbar_init(bLast, 1);
         for (uint32_t s = 0; s < 2; ++s) { mbar_init(bAccFull + 8 * s, 1); mbar_init(bAccEmpty + 8 * s, TG_EPI_WARPS); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -784,30 +789,29 @@ k_tensor_gemm(const TensorDesc* __restrict__ desc, const TensorSec* __restrict__
             const uint32_t nblk = ntiles * TN_KB;
             uint32_t s = 0, ph = 0, issued = 0;
             for (; issued < nblk; ++issued) {
-                ok = mbar_wait(bEmpty + 8 * s, ph ^ 1);
+                ok = mbar_wait(bEmpty + 8 * s, ph ^ 1, wait_ns);
                 if (!ok) break;
                 mbar_expect(bFull + 8 * s, TG_A_BYTES);
                 bulk_load(sA + s * TG_A_BYTES, src + (uint64_t)issued * TG_A_BYTES, TG_A_BYTES, bFull + 8 * s);
                 if (++s == TG_STAGES) { s = 0; ph ^= 1; }
             }
-            if (!ok) {
-                // the copies in flight end before the shared memory goes
-                mbar_wait(bConst, 0);
-                for (uint32_t k = issued > TG_STAGES ? issued - TG_STAGES : 0; k < issued; ++k)
-                    mbar_wait(bFull + 8 * (k % TG_STAGES), (k / TG_STAGES) & 1);
-            }
+            // the copies in flight end before the shared memory goes, whoever gave up
+            ok &= mbar_wait(bConst, 0, TG_DRAIN_NS);
+            for (uint32_t k = issued > TG_STAGES ? issued - TG_STAGES : 0; k < issued; ++k)
+                ok &= mbar_wait(bFull + 8 * (k % TG_STAGES), (k / TG_STAGES) & 1, TG_DRAIN_NS);
         }
     } else if (wid == TG_EPI_WARPS + 1) {
         if (lane == 0) {
-            ok = mbar_wait(bConst, 0);
+            ok = mbar_wait(bConst, 0, wait_ns);
             uint32_t s = 0, ph = 0;
+            bool issued = false;
             for (uint32_t t = 0; t < ntiles && ok; ++t) {
                 const uint32_t buf = t & 1;
-                ok = mbar_wait(bAccEmpty + 8 * buf, ((t >> 1) & 1) ^ 1);
+                ok = mbar_wait(bAccEmpty + 8 * buf, ((t >> 1) & 1) ^ 1, wait_ns);
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 for (uint32_t kb = 0; kb < TN_KB; ++kb) {
-                    ok = mbar_wait(bFull + 8 * s, ph);
+                    ok = mbar_wait(bFull + 8 * s, ph, wait_ns);
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint64_t da = smem_desc(sA + s * TG_A_BYTES), db = smem_desc(sB + kb * TG_B_BYTES);
@@ -815,9 +819,16 @@ k_tensor_gemm(const TensorDesc* __restrict__ desc, const TensorSec* __restrict__
                     for (uint32_t k = 0; k < 4; ++k)       // 32 bytes of K each
                         mma_i8(tmem + buf * TN_N, da + 2 * k, db + 2 * k, TG_IDESC, (kb | k) != 0);
                     mma_commit(bEmpty + 8 * s);
+                    issued = true;
                     if (++s == TG_STAGES) { s = 0; ph ^= 1; }
                 }
                 if (ok) mma_commit(bAccFull + 8 * buf);
+            }
+            // the matrix instructions end before the tensor memory goes (the epilogue,
+            // which waits for the last tile, may have given up)
+            if (issued) {
+                mma_commit(bLast);
+                ok &= mbar_wait(bLast, 0, TG_DRAIN_NS);
             }
         }
     } else {
@@ -850,7 +861,7 @@ k_tensor_gemm(const TensorDesc* __restrict__ desc, const TensorSec* __restrict__
             for (uint32_t r = 0; r < RH; ++r) P[r] = res_of<L>(ones[(d.ct0 + it.tile) * RT + (r < live ? r0 + r : 0)]);
             for (uint32_t k = 0; k < tn; ++k, ++t) {
                 const uint32_t buf = t & 1;
-                ok = mbar_wait(bAccFull + 8 * buf, (t >> 1) & 1);
+                ok = mbar_wait(bAccFull + 8 * buf, (t >> 1) & 1, wait_ns);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -1114,20 +1125,20 @@ void launch_tensor_consts(int L, const TensorDesc* d, uint32_t ntask, uint32_t n
 template <int L, int TAIL>
 static int gemm_l(uint32_t nitems, const TensorDesc* d, const TensorSec* sec, const TensorItem* items, const LaneRun* lr,
                   const RowInfo* info, const RowMod* mods, const uint8_t* w, const uint8_t* consts, const uint4* ones,
-                  void* part, uint32_t* err, cudaStream_t st) {
+                  void* part, uint32_t* err, uint64_t wait_ns, cudaStream_t st) {
     if (cudaFuncSetAttribute(k_tensor_gemm<L, TAIL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TG_SMEM) !=
         cudaSuccess)
         return -1;
     k_tensor_gemm<L, TAIL><<<nitems, TG_THREADS, TG_SMEM, st>>>(d, sec, items, lr, info, mods, w, consts, ones,
-                                                                (typename PartOf<L>::T*)part, err);
+                                                                (typename PartOf<L>::T*)part, err, wait_ns);
     return 0;
 }
 int launch_tensor_gemm(int L, uint32_t nitems, const TensorDesc* d, const TensorSec* sec, const TensorItem* items,
                        const LaneRun* lr, const RowMod* mods, const uint8_t* w, const uint8_t* consts,
-                       const uint4* ones, void* part, uint32_t* err, cudaStream_t st) {
-    if (L == 2) return gemm_l<2, 0>(nitems, d, sec, items, lr, nullptr, mods, w, consts, ones, part, err, st);
-    if (L == 3) return gemm_l<3, 0>(nitems, d, sec, items, lr, nullptr, mods, w, consts, ones, part, err, st);
-    return gemm_l<4, 0>(nitems, d, sec, items, lr, nullptr, mods, w, consts, ones, part, err, st);
+                       const uint4* ones, void* part, uint32_t* err, uint64_t wait_ns, cudaStream_t st) {
+    if (L == 2) return gemm_l<2, 0>(nitems, d, sec, items, lr, nullptr, mods, w, consts, ones, part, err, wait_ns, st);
+    if (L == 3) return gemm_l<3, 0>(nitems, d, sec, items, lr, nullptr, mods, w, consts, ones, part, err, wait_ns, st);
+    return gemm_l<4, 0>(nitems, d, sec, items, lr, nullptr, mods, w, consts, ones, part, err, wait_ns, st);
 }
 void launch_tensor_tail_build(const TensorDesc* d, const TensorSec* sec, uint32_t nsec, uint32_t nmt, uint8_t* w,
                               cudaStream_t st) {
@@ -1135,10 +1146,10 @@ void launch_tensor_tail_build(const TensorDesc* d, const TensorSec* sec, uint32_
 }
 int launch_tensor_tail_gemm(int L, uint32_t nitems, const TensorDesc* d, const TensorSec* sec, const TensorItem* items,
                             const RowInfo* info, const RowMod* mods, const uint8_t* w, const uint8_t* consts,
-                            const uint4* ones, void* part, uint32_t* err, cudaStream_t st) {
-    if (L == 2) return gemm_l<2, 1>(nitems, d, sec, items, nullptr, info, mods, w, consts, ones, part, err, st);
-    if (L == 3) return gemm_l<3, 1>(nitems, d, sec, items, nullptr, info, mods, w, consts, ones, part, err, st);
-    return gemm_l<4, 1>(nitems, d, sec, items, nullptr, info, mods, w, consts, ones, part, err, st);
+                            const uint4* ones, void* part, uint32_t* err, uint64_t wait_ns, cudaStream_t st) {
+    if (L == 2) return gemm_l<2, 1>(nitems, d, sec, items, nullptr, info, mods, w, consts, ones, part, err, wait_ns, st);
+    if (L == 3) return gemm_l<3, 1>(nitems, d, sec, items, nullptr, info, mods, w, consts, ones, part, err, wait_ns, st);
+    return gemm_l<4, 1>(nitems, d, sec, items, nullptr, info, mods, w, consts, ones, part, err, wait_ns, st);
 }
 template <int L>
 static void tail_rows_l(const TensorDesc* d, const TensorSec* sec, uint32_t ntask, uint32_t nblocks, const RowInfo* info,

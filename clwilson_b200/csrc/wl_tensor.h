@@ -33,7 +33,7 @@ constexpr uint32_t TN_SEG = 64;         // slots per segment of the label fold
 __host__ __device__ constexpr uint32_t tn_rows(int L) { return TN_N / (4u * (uint32_t)L); }
 
 // Where the rows live: their moduli, the accumulators to multiply into, and a
-// word that a kernel sets when one of its waits runs out.
+// word that a kernel sets when one of its waits runs out (after wl_ctx::wait_ns).
 struct TensorTarget {
     const RowMod* mods;
     uint4* acc;
@@ -109,7 +109,7 @@ void launch_tensor_consts(int L, const TensorDesc* d, uint32_t ntask, uint32_t n
 int launch_tensor_gemm(int L, uint32_t nitems, const TensorDesc* d, const TensorSec* sec, const TensorItem* items,
                        const LaneRun* lr, const RowMod* mods,
                        const uint8_t* w, const uint8_t* consts, const uint4* ones, void* part, uint32_t* err,
-                       cudaStream_t st);
+                       uint64_t wait_ns, cudaStream_t st);
 // tails: group products, the matrix product with each row's own number of groups
 // (items: cb0 = 0, ncb = group tiles), and the rest of each row's integers with
 // the product into acc
@@ -117,7 +117,7 @@ void launch_tensor_tail_build(const TensorDesc* d, const TensorSec* sec, uint32_
                               cudaStream_t st);
 int launch_tensor_tail_gemm(int L, uint32_t nitems, const TensorDesc* d, const TensorSec* sec, const TensorItem* items,
                             const RowInfo* info, const RowMod* mods, const uint8_t* w, const uint8_t* consts,
-                            const uint4* ones, void* part, uint32_t* err, cudaStream_t st);
+                            const uint4* ones, void* part, uint32_t* err, uint64_t wait_ns, cudaStream_t st);
 void launch_tensor_tail_rows(int L, const TensorDesc* d, const TensorSec* sec, uint32_t ntask, uint32_t nblocks,
                              const RowInfo* info, const RowMod* mods, const uint4* ones, const void* part, uint4* acc,
                              cudaStream_t st);

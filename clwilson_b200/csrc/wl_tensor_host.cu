@@ -365,7 +365,7 @@ int Products::chunk(const TensorTask* ts, size_t i0, size_t i1) {
         launch_tensor_consts(L, dd, nt, ntile, mods, as<uint8_t>(tb.consts), as<uint4>(tb.ones), st);
         if (launch_tensor_gemm(L, (uint32_t)items.size(), dd, ds, (const TensorItem*)(base + o_item), dr, mods,
                                as<uint8_t>(tb.w), as<uint8_t>(tb.consts), as<uint4>(tb.ones), tb.part.p,
-                               to.err, st))
+                               to.err, c->wait_ns, st))
             return WL_ERR_CUDA;
         launch_tensor_fold(L, dd, nt, fold_blk, as<FoldSeg>(tb.segs), mods, tb.part.p, tb.seg.p, st);
         launch_tensor_combine(L, dd, nt, row_blk, max_blocks, as<uint32_t>(tb.lab_seg), mods, as<uint4>(tb.ones),
@@ -510,7 +510,7 @@ int tensor_tails(wl_ctx* c, const std::vector<TensorTail>& tails, const std::vec
         if (!items.empty() &&
             launch_tensor_tail_gemm(L, (uint32_t)items.size(), dd, ds, (const TensorItem*)(base + o_item),
                                     as<RowInfo>(c->rowinfo), to.mods, as<uint8_t>(tb.w), as<uint8_t>(tb.consts),
-                                    as<uint4>(tb.ones), tb.part.p, to.err, st))
+                                    as<uint4>(tb.ones), tb.part.p, to.err, c->wait_ns, st))
             return WL_ERR_CUDA;
         launch_tensor_tail_rows(L, dd, ds, nt, row_blk, as<RowInfo>(c->rowinfo), to.mods, as<uint4>(tb.ones), tb.part.p,
                                 to.acc, st);

@@ -190,6 +190,13 @@ int wl_rows_product_parts(wl_ctx *ctx, size_t n, const uint64_t *p, size_t npart
 /* Forget the resident column table; the next call sieves it again. */
 void wl_drop_columns(wl_ctx *ctx);
 
+/* Limit in nanoseconds of each wait inside the tensor-core products' kernels
+ * (4 s when the context is opened; such a wait takes microseconds).  A call
+ * one of whose waits runs out ends with WL_ERR_CUDA and the context stays
+ * usable.  With 0 every wait runs out at once, which shows a caller its
+ * handling of that error. */
+int wl_set_wait_limit(wl_ctx *ctx, uint64_t ns);
+
 /* Column product of one class without any device allocation.
  *
  * No counterpart in the reference.  For callers that cannot allocate device
