@@ -131,7 +131,8 @@ SYMBOLS = ("wl_open", "wl_close", "wl_strerror", "wl_stream", "wl_check_range", 
            "wl_probe",
            "wl_column_product_noalloc", "wl_get_tuning", "wl_set_tuning", "wl_autotune",
            "wl_server_open", "wl_server_submit", "wl_server_poll", "wl_server_wait", "wl_server_results",
-           "wl_server_rows", "wl_server_cancel", "wl_server_release", "wl_server_stats_get", "wl_server_close")
+           "wl_server_rows", "wl_server_cancel", "wl_server_release", "wl_server_stats_get",
+           "wl_server_set_wait_limit", "wl_server_close")
 # cellL: the carry-chain cell; cellLw: the wide-product cell the sweeps run by default
 PROBES = {"mad": 0, "madhi": 1, "cell2": 2, "cell3": 3, "cell4": 4, "madwide": 5,
           "cell2w": 101, "cell3w": 111, "cell4w": 121}
@@ -197,8 +198,10 @@ def load_library(path: str = LIB_PATH):
     L.wl_server_cancel.argtypes = [vp, u64]
     L.wl_server_release.argtypes = [vp, u64]
     L.wl_server_stats_get.argtypes = [vp, ctypes.POINTER(_ServerStats)]
+    L.wl_server_set_wait_limit.argtypes = [vp, u64]
     for fn in ("wl_server_open", "wl_server_submit", "wl_server_poll", "wl_server_wait", "wl_server_results",
-               "wl_server_rows", "wl_server_cancel", "wl_server_release", "wl_server_stats_get"):
+               "wl_server_rows", "wl_server_cancel", "wl_server_release", "wl_server_stats_get",
+               "wl_server_set_wait_limit"):
         getattr(L, fn).restype = ctypes.c_int
     L.wl_server_close.argtypes = [vp]
     L.wl_server_close.restype = None
@@ -586,6 +589,12 @@ class Server:
         rc = self._L.wl_server_release(self._srv, rid)
         if rc:
             raise WilsonError(rc, "wl_server_release")
+
+    def set_wait_limit(self, ns: int) -> None:
+        """As Engine.set_wait_limit, from the next step on."""
+        rc = self._L.wl_server_set_wait_limit(self._srv, ns)
+        if rc:
+            raise WilsonError(rc, "wl_server_set_wait_limit")
 
     def stats(self) -> dict:
         st = _ServerStats()

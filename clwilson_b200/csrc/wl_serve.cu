@@ -112,6 +112,7 @@ struct wl_server {
     uint32_t shares = WL_SHARES_LEAST_WORK;
     DevBuf info, mods, acc, out, pbuckets, bdef, ipart;
     uint32_t* terr = nullptr;                  // error word of the tensor-core products (behind bdef)
+    int step_err = 0;                          // a completed step's error: its rows are not to be used
     size_t tbudget = 0;                        // workspace they may take (0: none, the sweeps run)
     bool tbudget_known = false;                // asked for at the first admission
     // Two sets of a step's buffers: the scheduler plans and queues step k+1
@@ -826,16 +827,20 @@ static void serve_retire(wl_server* s, SReq* q, int state, int rc) {
 }
 
 // Waits for the step in `sl`, takes its device time, and completes the
-// requests whose lift followed it.  err != 0 (a failed step) fails them.
+// requests whose lift followed it.  err != 0 (a failed step) fails them.  A
+// step whose tensor-core products set their error word may have multiplied any
+// running request's rows by anything, also of requests that finish in later
+// steps: step_err fails what completes from here on, and serve_recover the rest.
 static void serve_complete(wl_server* s, wl_server::Slot& sl, int err = 0) {
     if (!sl.inflight) return;
     const double t = s->now_ms();
+    if (!err) err = s->step_err;
     if (!err && cudaEventSynchronize(sl.e1) != cudaSuccess) err = WL_ERR_CUDA;
     if (!err && sl.tensor) {
         uint32_t ran_out = 0;
         if (cudaMemcpyAsync(&ran_out, s->terr, 4, cudaMemcpyDeviceToHost, s->c->st3) != cudaSuccess ||
             cudaStreamSynchronize(s->c->st3) != cudaSuccess || ran_out)
-            err = WL_ERR_CUDA;
+            err = s->step_err = WL_ERR_CUDA;
     }
     sl.tensor = false;
     if (!err) {
@@ -860,9 +865,21 @@ static void serve_drain(wl_server* s, int err = 0) {
     if (err) cudaGetLastError();
 }
 
+// After a failed step: every request still running fails with its code, and
+// the session starts afresh with the next one.
+static void serve_recover(wl_server* s, int err) {
+    serve_drain(s, err);
+    const std::vector<SReq*> all(s->active);
+    for (SReq* q : all) serve_retire(s, q, WL_REQ_FAILED, err);
+    cudaStreamSynchronize(s->c->st);             // nothing that may set the error word is left
+    cudaMemset(s->terr, 0, 4);
+    s->step_err = 0;
+}
+
 static void serve_loop(wl_server* s) {
     cudaSetDevice(s->c->device);
     while (true) {
+        if (s->step_err) serve_recover(s, s->step_err);
         // queued requests to admit (cancelled ones end here), and cancelled active ones
         std::vector<SReq*> cands, cancelled;
         {
@@ -895,6 +912,7 @@ static void serve_loop(wl_server* s) {
         if (!cands.empty()) {
             // admission synchronises the stream and may grow the column table
             serve_drain(s);
+            if (s->step_err) serve_recover(s, s->step_err);
             std::vector<int> res;
             const double t = s->now_ms();
             serve_admit_batch(s, cands, res);
@@ -925,14 +943,12 @@ static void serve_loop(wl_server* s) {
         for (SReq* q : s->active) work |= !q->finishing && !q->cancel_seen;
         if (work) {
             serve_complete(s, s->slot[s->cur]);
+            if (s->step_err) continue;
             const double t = s->now_ms();
             const int e = serve_step(s);
             s->ws.ms_wall_steps += s->now_ms() - t;
             if (e) {
-                // a failed step: every request still running fails with its code
-                serve_drain(s, e);
-                std::vector<SReq*> all(s->active);
-                for (SReq* q : all) serve_retire(s, q, WL_REQ_FAILED, e);
+                serve_recover(s, e);
                 continue;
             }
         }
@@ -1129,6 +1145,11 @@ int wl_server_release(wl_server* s, uint64_t id) {
     delete q;
     s->reqs.erase(id);
     return 0;
+}
+
+int wl_server_set_wait_limit(wl_server* s, uint64_t ns) {
+    if (!s) return WL_ERR_ARG;
+    return wl_set_wait_limit(s->c, ns);
 }
 
 int wl_server_stats_get(wl_server* s, wl_server_stats* st) {

@@ -357,6 +357,10 @@ int wl_server_cancel(wl_server *srv, uint64_t id);
 /* Forget an ended request (its id becomes invalid). */
 int wl_server_release(wl_server *srv, uint64_t id);
 int wl_server_stats_get(wl_server *srv, wl_server_stats *stats);
+/* As wl_set_wait_limit, for the session's steps from the next one on.  A wait
+ * that runs out ends every request then running with WL_REQ_FAILED and
+ * WL_ERR_CUDA; the session goes on with later ones. */
+int wl_server_set_wait_limit(wl_server *srv, uint64_t ns);
 /* Stop the scheduler (running requests are abandoned) and free the server. */
 void wl_server_close(wl_server *srv);
 
