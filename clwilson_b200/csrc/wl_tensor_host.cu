@@ -62,8 +62,6 @@ void task_digits(const TensorTask& t, uint32_t* w, uint32_t* nwin) {
 
 uint32_t row_tiles_of(uint32_t nrows, int L) { return (nrows + tn_rows(L) - 1) / tn_rows(L); }
 
-// Shares of the workspace: group lists and products together, lane-run
-// products, row constants.  Tasks are cut so that a chunk keeps within them.
 // A buffer that must grow grows by half, so that calls and steps of slowly rising
 // size do not free and allocate each time.
 int grow(TensorBufs& tb, DevBuf& b, size_t bytes) {
@@ -108,8 +106,15 @@ int first_block(TensorBufs& tb) {
     return 0;
 }
 
+// Shares of the workspace: list entries (4 bytes each), group tiles (64 KB each;
+// where tasks are many and small, most of them padding), and the bytes of the
+// lane-run products and of the row constants.  Buckets are cut into pieces and
+// rows into slabs so that a task keeps within them, and a chunk takes as many
+// tasks as keep within them together: with the folded products, which are never
+// more than the lane runs', a chunk holds about 1.2 GB at most.  Buffers that grew by
+// half may be half as large again.
 struct Limits {
-    double entries, part, consts;
+    double entries, tiles, part, consts;
 };
 constexpr uint32_t WAVE_TASKS = 1024;      // tasks counted in one launch
 
@@ -128,6 +133,7 @@ class Products {
 public:
     Products(wl_ctx* c, const TensorTarget& to, size_t budget) : c(c), tb(c->tb), to(to) {
         lim.entries = std::min<double>((double)budget / 2 / 9.0, (double)(1u << 25));
+        lim.tiles = std::min<double>((double)budget * 3 / 8, 402e6) / (double)(TN_M * TN_K);
         lim.part = std::min<double>((double)budget / 4, 256e6);
         lim.consts = std::min<double>((double)budget / 4, 128e6);
     }
@@ -241,7 +247,9 @@ int Products::wave(size_t t0, size_t t1) {
             const double pe = (double)z.slots * tiles * tn_rows(t.L) * (t.L == 2 ? 8 : 16);
             const double ke = (double)tiles * TN_N * TN_K;
             const bool whole = rows >= t.nrows;     // a task in several slabs goes alone
-            if (j > i && (!whole || e + (double)z.entries > lim.entries || p + pe > lim.part || k + ke > lim.consts)) break;
+            if (j > i && (!whole || e + (double)z.entries > lim.entries || (double)(mt + group_tiles(z)) > lim.tiles ||
+                          p + pe > lim.part || k + ke > lim.consts))
+                break;
             e += (double)z.entries;
             p += pe;
             k += ke;
@@ -443,15 +451,24 @@ int tensor_products(wl_ctx* c, std::vector<TensorTask> tasks, const TensorTarget
     return p.run();
 }
 
-// The tails of buckets of one limb width, a slab of rows at a time: row tiles
-// need whole group tiles only up to their last row's end (rows are in ascending
-// p, so ascending Tp).
+// The tails of buckets, a slab of rows at a time: TAIL_TILES row tiles (128 MB of
+// constants) with the groups that the slab's last row needs.  Rows are in ascending
+// p, so ascending Tp, and a row tile needs whole group tiles only up to its last
+// row's end.  One launch takes slabs of one limb width, of several tails where they
+// are small, that keep within TAIL_TILES and 128 MB of groups together.
 int tensor_tails(wl_ctx* c, const std::vector<TensorTail>& tails, const std::vector<RowInfo>& ri, const TensorTarget& to) {
+    constexpr uint32_t TAIL_TILES = 1024, TAIL_GROUP_TILES = 2048;
     cudaStream_t st = c->st;
     TensorBufs& tb = c->tb;
     RC(first_block(tb));
-    for (size_t i0 = 0; i0 < tails.size();) {
-        const int L = (int)tails[i0].L;
+    std::vector<TensorTail> slabs;
+    for (const TensorTail& t : tails) {
+        const uint32_t step = TAIL_TILES * tn_rows((int)t.L);
+        for (uint32_t r0 = 0; r0 < t.nrows; r0 += step)
+            slabs.push_back({ t.T, t.row_begin + r0, std::min(step, t.nrows - r0), t.L });
+    }
+    for (size_t i0 = 0; i0 < slabs.size();) {
+        const int L = (int)slabs[i0].L;
         const uint32_t rt = tn_rows(L);
         std::vector<TensorDesc> dc;
         std::vector<TensorSec> secs;
@@ -459,14 +476,13 @@ int tensor_tails(wl_ctx* c, const std::vector<TensorTail>& tails, const std::vec
         uint32_t ntile = 0, nmt = 0, row_blk = 0;
         uint64_t part = 0;
         size_t i1 = i0;
-        // as many tails as keep the constants within 128 MB and the groups within as much
-        for (; i1 < tails.size() && (int)tails[i1].L == L; ++i1) {
-            const TensorTail& t = tails[i1];
+        for (; i1 < slabs.size() && (int)slabs[i1].L == L; ++i1) {
+            const TensorTail& t = slabs[i1];
             const uint64_t last = ri[t.row_begin + t.nrows - 1].Tp;
             const double k = 511.99 / std::log2((double)last + 2.0);
             const uint32_t g = 8 * (uint32_t)std::min<double>(k, (double)TN_GMAX / 8), tiles = row_tiles_of(t.nrows, L);
             const uint64_t mts = ((last - t.T) / g + TN_M - 1) / TN_M;
-            if (i1 > i0 && (ntile + tiles > 1024 || nmt + mts > 2048)) break;
+            if (i1 > i0 && (ntile + tiles > TAIL_TILES || nmt + mts > TAIL_GROUP_TILES)) break;
             TensorDesc d;
             memset(&d, 0, sizeof(d));
             d.T = t.T;
