@@ -611,7 +611,7 @@ static int run_ranges(wl_ctx* c, const wl_range* ranges, size_t nr, uint64_t qca
     std::vector<TensorTask> tensor;
     std::vector<char> on_tensor(nb, 0);
     size_t tbudget = 0;
-    if (tensor_enabled()) {
+    if (c->tensor) {
         // all buckets on one path, or, where both have work, each on its faster one
         double all_tensor = TENSOR_CALL_MS, all_sweeps = SWEEP_CALL_MS, mixed = TENSOR_CALL_MS + SWEEP_CALL_MS,
                entries = 0;
@@ -1161,6 +1161,7 @@ int wl_open(int device, wl_ctx** out) {
     if (cudaSetDevice(device) != cudaSuccess) { delete c; return WL_ERR_CUDA; }
     cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, device);
     if (const char* v = getenv("WL_CELL_VARIANT")) c->cell_variant = atoi(v);
+    if (const char* v = getenv("WL_TENSOR")) c->tensor = atoi(v) != 0;
     default_tuning(c);
     if (cudaStreamCreateWithFlags(&c->st, cudaStreamNonBlocking) != cudaSuccess ||
         cudaStreamCreateWithFlags(&c->st2, cudaStreamNonBlocking) != cudaSuccess ||

@@ -164,6 +164,8 @@ struct wl_ctx {
     DevBuf work;         // dense sweep work counters: column cells, window cells, products; then the
                          // tensor-core product's error word
     TensorBufs tb;
+    bool tensor = true;  // false: every bucket and tail takes the sweeps (WL_TENSOR=0 in the environment when
+                         // the context is opened)
 };
 
 // Every prime below `limit` (<= 2^32) in the context's resident column table.
@@ -190,11 +192,6 @@ int gen_test_primes(wl_ctx* c, const wl_range* ranges, size_t nr, std::vector<Ra
                     std::vector<uint64_t>& tps, bool allow_empty = false);
 // Frees the tensor-core products' workspace.
 void tensor_release(wl_ctx* c);
-// WL_TENSOR=0 in the environment turns the tensor-core products off, for comparisons.
-inline bool tensor_enabled() {
-    static const bool off = getenv("WL_TENSOR") && atoi(getenv("WL_TENSOR")) == 0;
-    return !off;
-}
 // Workspace the tensor-core products may take for about `entries` list entries
 // and `rows` rows; 0: too little memory, the sweeps run instead.
 size_t tensor_budget(wl_ctx* c, double entries, double rows);

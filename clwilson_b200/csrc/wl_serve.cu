@@ -213,7 +213,7 @@ static void serve_admit_batch(wl_server* s, const std::vector<SReq*>& cands, std
     result.assign(nc, 1);
     if (!s->tbudget_known) {
         s->tbudget_known = true;
-        if (tensor_enabled()) s->tbudget = tensor_budget(c, 1e9, 1e6);   // what a large step would take
+        if (c->tensor) s->tbudget = tensor_budget(c, 1e9, 1e6);   // what a large step would take
     }
     cudaEventRecord(s->e0, c->st);
     // 1. test primes of the candidates that have none yet
