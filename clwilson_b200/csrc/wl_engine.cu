@@ -1354,10 +1354,20 @@ int wl_set_tuning(wl_ctx* c, const wl_tuning* t) {
     return 0;
 }
 
+// The sweeps alone, whatever route the context takes otherwise: their kernels are
+// what the tuning chooses among.
+struct SweepsOnly {
+    wl_ctx* c;
+    const bool keep;
+    explicit SweepsOnly(wl_ctx* c) : c(c), keep(c->tensor) { c->tensor = false; }
+    ~SweepsOnly() { c->tensor = keep; }
+};
+
 // One tuning measurement: the sweep-phase device time of the sample (best of
 // `reps` runs) and a digest of its rows, which every candidate must reproduce.
 static int tune_time(wl_ctx* c, const wl_range* r, size_t nr, uint64_t qcap, int reps, double* ms,
                      uint64_t* digest) {
+    const SweepsOnly sweeps(c);
     double best = 1e300;
     for (int rep = 0; rep < reps; ++rep) {
         RunOut ro;

@@ -165,7 +165,7 @@ struct wl_ctx {
                          // tensor-core product's error word
     TensorBufs tb;
     bool tensor = true;  // false: every bucket and tail takes the sweeps (WL_TENSOR=0 in the environment when
-                         // the context is opened)
+                         // the context is opened; while the sweeps' kernels are timed for tuning)
 };
 
 // Every prime below `limit` (<= 2^32) in the context's resident column table.

@@ -266,7 +266,9 @@ int wl_get_tuning(wl_ctx *ctx, wl_tuning *out);
 int wl_set_tuning(wl_ctx *ctx, const wl_tuning *t);
 /* Time the variants and keep the fastest in the context, by coordinate
  * descent (prefix-fold sweep, dense sweep, merge fan-in; a candidate must be
- * more than 2% faster to replace the current choice).  ranges/n/q_cap: the
+ * more than 2% faster to replace the current choice).  The samples run on the
+ * sweeps alone, also where a call would take the tensor-core products; the
+ * choice holds for the work that the sweeps keep.  ranges/n/q_cap: the
  * workload to tune on (one choice for all its limb widths); n = 0: built-in
  * samples, one per L with bit (L - 2) set in limbs_mask (0: all), a few
  * seconds each.  Every candidate must produce the same rows; a mismatch

@@ -144,3 +144,21 @@ def test_session_on_the_sweeps(eng, engine):
             assert srv.wait(rid, 600_000).state == "done"
             want, st = engine.rows(lo, hi, q_cap=q)
             _same(srv.rows(rid), want)
+
+
+def test_tuning_times_the_sweeps(engine):
+    # what autotune reports for a caller's ranges is the sweeps' time, here tens of
+    # times that of the call itself
+    r, q = (TOP - 50000, TOP), 1 << 24
+    with sweeps_alone():
+        e = wl.Engine(0)
+    with e:
+        e.rows(*r, q_cap=q)
+        sweeps = min(e.rows(*r, q_cap=q)[1].ms_sweep for _ in range(3))
+    with wl.Engine(0) as e:
+        e.rows(*r, q_cap=q)
+        call = min(e.rows(*r, q_cap=q)[1].ms_sweep for _ in range(3))
+        assert call < sweeps / 5
+        t = e.autotune([r], q_cap=q)
+        assert t["ms"][2] > sweeps / 2
+        assert e.rows(*r, q_cap=q)[1].tensor_macs > 0          # the context's own route is back
