@@ -497,9 +497,10 @@ static int count_columns(wl_ctx* c, const std::vector<uint64_t>& keys, std::vect
 
 // Columns q in [q_lo, q_cap) (q_cap = 0: through the class target, then the
 // tail and the lift); init: the rows' running products before q_lo, two
-// digits (s0, s1) per row in output order, or NULL for 1.
-static int run_ranges(wl_ctx* c, const wl_range* ranges, size_t nr, uint64_t qcap, RunOut& out, wl_stats* st,
-                      uint64_t q_lo = 2, const uint64_t* init = nullptr, bool graph = false) {
+// digits (s0, s1) per row in output order, or NULL for 1.  lean: the sweeps
+// alone, in splits whose products fit the free memory.
+static int run_ranges_once(wl_ctx* c, const wl_range* ranges, size_t nr, uint64_t qcap, RunOut& out, wl_stats* st,
+                           uint64_t q_lo, const uint64_t* init, bool graph, bool lean) {
     const bool full = (qcap == 0);
     c->launches = 0;
     c->h2d = c->d2h = 0;
@@ -611,7 +612,7 @@ static int run_ranges(wl_ctx* c, const wl_range* ranges, size_t nr, uint64_t qca
     std::vector<TensorTask> tensor;
     std::vector<char> on_tensor(nb, 0);
     size_t tbudget = 0;
-    if (c->tensor) {
+    if (c->tensor && !lean) {
         // all buckets on one path, or, where both have work, each on its faster one
         double all_tensor = TENSOR_CALL_MS, all_sweeps = SWEEP_CALL_MS, mixed = TENSOR_CALL_MS + SWEEP_CALL_MS,
                entries = 0;
@@ -682,10 +683,11 @@ static int run_ranges(wl_ctx* c, const wl_range* ranges, size_t nr, uint64_t qca
     }
     double scale = 1.0;
     {
-        // 256 MiB of partials always fit: no need to ask for the free memory
-        const double always = (double)(256ull << 20) / 16.0;
-        scale = split_scale(sbs, W, target_threads, always);
-        if (scale < 1.0) {
+        // up to 256 MiB of partials nearly always fit: the free memory is not asked for
+        // then, and where they do not the call starts over (lean)
+        const double unasked = (double)(256ull << 20) / 16.0;
+        scale = split_scale(sbs, W, target_threads, unasked);
+        if (scale < 1.0 || lean) {
             const double budget =
                 std::min<double>((double)(free_memory() + c->part.cap) / 3.0, 24.0 * (1ull << 30)) / 16.0;
             scale = split_scale(sbs, W, target_threads, budget);
@@ -1063,6 +1065,18 @@ static int run_ranges(wl_ctx* c, const wl_range* ranges, size_t nr, uint64_t qca
         st->tensor_macs = c->tensor_macs;
     }
     return 0;
+}
+
+// As run_ranges_once.  Where device memory ran out, the call runs once more without
+// the tensor-core products, whose workspace is given back first.
+static int run_ranges(wl_ctx* c, const wl_range* ranges, size_t nr, uint64_t qcap, RunOut& out, wl_stats* st,
+                      uint64_t q_lo = 2, const uint64_t* init = nullptr, bool graph = false) {
+    const int rc = run_ranges_once(c, ranges, nr, qcap, out, st, q_lo, init, graph, false);
+    if (rc != WL_ERR_NOMEM) return rc;
+    for (cudaStream_t s : { c->st, c->st2, c->st3 }) CK(cudaStreamSynchronize(s));
+    tensor_release(c);
+    out = RunOut();
+    return run_ranges_once(c, ranges, nr, qcap, out, st, q_lo, init, graph, true);
 }
 
 // results.txt value of one row (cl_wilson.cpp:872-898): 1 if it is a result line

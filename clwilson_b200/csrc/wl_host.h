@@ -201,8 +201,10 @@ size_t tensor_budget(wl_ctx* c, double entries, double rows);
 double tensor_times(uint32_t nrows, int L, uint64_t T, uint64_t c0, uint64_t nsparse, uint64_t ndense, double* tensor,
                     double* sweeps);
 // Multiplies each task's columns into its rows' accumulators, on the main
-// stream (it waits once for the stream).
-int tensor_products(wl_ctx* c, std::vector<wl::TensorTask> tasks, const wl::TensorTarget& to, size_t budget);
+// stream (it waits once for the stream).  done: the first column of each task that
+// is not multiplied in, which after WL_ERR_NOMEM may lie anywhere in the task.
+int tensor_products(wl_ctx* c, std::vector<wl::TensorTask> tasks, const wl::TensorTarget& to, size_t budget,
+                    std::vector<uint64_t>* done = nullptr);
 // Multiplies the rows' consecutive-integer tails T+1 .. Tp into their
 // accumulators, on the main stream; c->rowinfo holds the rows ri.
 int tensor_tails(wl_ctx* c, const std::vector<wl::TensorTail>& tails, const std::vector<wl::RowInfo>& ri,

@@ -115,6 +115,7 @@ struct wl_server {
     int step_err = 0;                          // a completed step's error: its rows are not to be used
     size_t tbudget = 0;                        // workspace they may take (0: none, the sweeps run)
     bool tbudget_known = false;                // asked for at the first admission
+    bool short_of_memory = false;              // the products' workspace did not fit: asked for again once idle
     // Two sets of a step's buffers: the scheduler plans and queues step k+1
     // into one set while step k still runs on the other, and completes step k
     // (its timing, the requests whose lift followed it) meanwhile.
@@ -211,8 +212,9 @@ static void serve_admit_batch(wl_server* s, const std::vector<SReq*>& cands, std
     wl_ctx* c = s->c;
     const size_t nc = cands.size();
     result.assign(nc, 1);
-    if (!s->tbudget_known) {
+    if (!s->tbudget_known || (s->short_of_memory && s->active.empty())) {
         s->tbudget_known = true;
+        s->short_of_memory = false;
         if (c->tensor) s->tbudget = tensor_budget(c, 1e9, 1e6);   // what a large step would take
     }
     cudaEventRecord(s->e0, c->st);
@@ -686,9 +688,23 @@ static int serve_step(wl_server* s) {
     if (!tensor.empty()) {
         // waits for the step before it; its own kernels then run beside the planning below
         const uint32_t before = c->launches;
-        RC(tensor_products(c, tensor, { as<RowMod>(s->mods), as<uint4>(s->acc), s->terr }, s->tbudget));
+        std::vector<uint64_t> done;
+        const int rc = tensor_products(c, tensor, { as<RowMod>(s->mods), as<uint4>(s->acc), s->terr }, s->tbudget, &done);
         s->ws.launches += c->launches - before;
         sl.tensor = true;
+        if (rc == WL_ERR_NOMEM) {
+            // no room for their workspace: the sweeps take every bucket from where the
+            // products got to, from the next step on
+            tensor_release(c);
+            s->tbudget = 0;
+            s->short_of_memory = true;
+            for (SBucket& b : s->sb) b.tcost = 0;
+            size_t k = 0;
+            for (Work& w : work)
+                if (w.kind == 3) w.len = done[k++] - w.c0;
+        } else {
+            RC(rc);
+        }
     }
     CK(cudaMemcpyAsync(sl.sbuckets.p, sbk.data(), sbk.size() * sizeof(Bucket), cudaMemcpyHostToDevice, c->st));
     sl.dirty_top = top;

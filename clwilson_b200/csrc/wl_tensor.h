@@ -16,6 +16,7 @@ struct TensorTask {
     uint32_t row_begin, nrows;
     int L;
     uint32_t q_max;      // bound on its largest column
+    uint32_t id = 0;     // the caller's place in its list (tensor_products sets it)
 };
 
 // Geometry of the tensor-core product (see wl_tensor.cu).

@@ -67,7 +67,7 @@ uint32_t row_tiles_of(uint32_t nrows, int L) { return (nrows + tn_rows(L) - 1) /
 int grow(TensorBufs& tb, DevBuf& b, size_t bytes) {
     if (bytes <= b.cap && b.p) return 0;
     const size_t want = std::max(bytes, b.cap + b.cap / 2);
-    if (!tb.pool) return ensure(b, want);
+    if (!tb.pool) return ensure(b, want) ? ensure(b, bytes) : 0;
     if (b.p && !b.inner) cudaFreeAsync(b.p, tb.st);
     b = DevBuf();
     for (size_t n : { want, bytes }) {
@@ -137,6 +137,7 @@ public:
         lim.part = std::min<double>((double)budget / 4, 256e6);
         lim.consts = std::min<double>((double)budget / 4, 128e6);
     }
+    std::vector<uint64_t>* done = nullptr;   // see tensor_products
     void add(const TensorTask& whole);
     int run();
 
@@ -278,7 +279,8 @@ int Products::wave(size_t t0, size_t t1) {
 }
 
 // Tasks [i0, i1) of the wave: their lists and group products once, then per
-// slab of rows the constants, the matrix product and the label folds.
+// slab of rows the constants, the matrix product and the label folds.  The first
+// slab is the largest, so that an allocation fails before any row is multiplied.
 int Products::chunk(const TensorTask* ts, size_t i0, size_t i1) {
     cudaStream_t st = c->st;
     const int L = ts[i0].L;
@@ -383,6 +385,8 @@ int Products::chunk(const TensorTask* ts, size_t i0, size_t i1) {
         first = false;
         if (nt > 1) break;
     }
+    if (done)
+        for (size_t i = i0; i < i1; ++i) (*done)[ts[i].id] = ts[i].c1;
     return 0;
 }
 
@@ -444,9 +448,16 @@ double tensor_times(uint32_t nrows, int L, uint64_t T, uint64_t c0, uint64_t nsp
     return entries;
 }
 
-int tensor_products(wl_ctx* c, std::vector<TensorTask> tasks, const TensorTarget& to, size_t budget) {
+int tensor_products(wl_ctx* c, std::vector<TensorTask> tasks, const TensorTarget& to, size_t budget,
+                    std::vector<uint64_t>* done) {
+    if (done) done->resize(tasks.size());
+    for (uint32_t i = 0; i < tasks.size(); ++i) {
+        tasks[i].id = i;
+        if (done) (*done)[i] = tasks[i].c0;
+    }
     std::stable_sort(tasks.begin(), tasks.end(), [](const TensorTask& a, const TensorTask& b) { return a.L < b.L; });
     Products p(c, to, budget);
+    p.done = done;
     for (const TensorTask& t : tasks) p.add(t);
     return p.run();
 }
