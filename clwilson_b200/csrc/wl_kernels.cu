@@ -1119,7 +1119,7 @@ k_finish(const Bucket* __restrict__ buckets, const RowInfo* __restrict__ info, c
          const uint4* __restrict__ ipart, uint32_t row_begin, uint32_t nrows, int full,
          RowOut* __restrict__ out, const uint4* __restrict__ acc1, const Deficit* __restrict__ def1,
          const uint4* __restrict__ acc2, const Deficit* __restrict__ def2, int merged) {
-    __shared__ uint32_t sv[5][L][32];              // T_p! mod n; 2^p, 3^p, 1/c (Montgomery form); c or a
+    __shared__ uint32_t sv[4][L][32];              // T_p! mod n; 2^p, 3^p, 1/c (Montgomery form)
     __shared__ int64_t su[32], sc[32];
     __shared__ uint64_t sd[2][32];
     __shared__ uint8_t sok[32];

@@ -1,6 +1,7 @@
 // wl_tensor_host.cu -- plans the tensor-core column products (wl_tensor.cu):
-// cuts the buckets into tasks that fit the workspace, reads the digit counts
-// back, lays the labels out in lane runs and launches the kernels.
+// cuts the buckets into tasks that fit the workspace, reads back what each takes
+// (the digits are counted and laid out in lane runs on the device) and launches
+// the kernels.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
