@@ -88,6 +88,8 @@ int ensure_columns(wl_ctx* c, uint64_t limit) {
     nl = (nl + SEG_SPAN - 1) / SEG_SPAN * SEG_SPAN;
     if (nl > top) nl = top;
     const uint32_t nseg = (uint32_t)(nl / SEG_SPAN);
+    // no table until the larger one is there: its buffer goes before the new one comes
+    wl_drop_columns(c);
     RC(ensure(c->bitmap, (size_t)nseg * SEG_WORDS * 4));
     RC(ensure(c->segcount, (size_t)nseg * 4));
     RC(ensure(c->offsets, (size_t)(nseg + 1) * 8));

@@ -169,6 +169,7 @@ struct wl_ctx {
 };
 
 // Every prime below `limit` (<= 2^32) in the context's resident column table.
+// After an error there may be no table (col_limit = 0).
 int ensure_columns(wl_ctx* c, uint64_t limit);
 // The column groups of the resident table for the prefix-fold sweep, built on
 // the main stream when first asked for after the table was; none (every column

@@ -308,7 +308,13 @@ static void serve_admit_batch(wl_server* s, const std::vector<SReq*>& cands, std
         }
     for (auto& a : adm)
         for (uint64_t key : a.keys) keys.push_back(key >= BIG_LO ? isqrt_floor(key) : 0);
+    const uint64_t had = c->col_limit;
     int e = ensure_columns(c, need);
+    if (e && c->col_limit < had) {
+        // the larger table did not come: back to the one that running requests read, or they fail
+        const int lost = ensure_columns(c, had);
+        if (lost) s->step_err = lost;
+    }
     if (!e) e = ensure(c->keys, keys.size() * 8);
     if (!e) e = ensure(c->counts, keys.size() * 8);
     if (e) { fail_admitted(e); return; }

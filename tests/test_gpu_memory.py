@@ -103,3 +103,47 @@ def test_session(expected):
         again = srv.submit(*CALLS[1])
         assert srv.wait(again, 600_000).state == "done"
         assert np.array_equal(srv.rows(again)["s1"], expected[CALLS[1]]["s1"])
+
+
+def test_column_table_that_does_not_fit():
+    # a table for 5e8 takes 110 MB: the call fails, and the smaller table that it was to
+    # replace is sieved again by the next call that needs it
+    small, large = (10**6, 10**6 + 2000), (10**9, 10**9 + 100)
+    with wl.Engine(0) as e:
+        want, _ = e.rows(*small)
+        with free_memory(30 * MB):
+            with pytest.raises(wl.WilsonError) as err:
+                e.rows(*large)
+            assert err.value.code == -8
+            rows, _ = e.rows(*small)
+            assert np.array_equal(rows, want)
+        rows, _ = e.rows(*large)
+        assert (rows["status"] == 0).all() and (rows["rem"] == 0).all()
+
+
+def test_session_whose_table_does_not_fit(expected):
+    # a request that needs the larger table fails; the one that is running, on the sweeps
+    # in small steps, goes on with the table that it was admitted with
+    lo, hi, q = 10**13, 10**13 + 200000, 1 << 27
+    with _engine(False) as e:
+        want, _ = e.rows(lo, hi, q_cap=q)
+    os.environ["WL_TENSOR"] = "0"
+    try:
+        srv = wl.Server(0, pool_bytes=64 * MB, step_cells=1 << 26)
+    finally:
+        os.environ.pop("WL_TENSOR")
+    with srv:
+        long = srv.submit(lo, hi, q)
+        while srv.poll(long).state == "queued":
+            pass
+        with free_memory(40 * MB):
+            large = srv.submit(10**9, 10**9 + 100)
+            info = srv.wait(large, 600_000)
+            assert info.state == "failed" and info.rc == -8
+            assert srv.poll(long).state == "active"
+            assert srv.wait(long, 600_000).state == "done"
+        got = srv.rows(long)
+        for f in ("p", "s0", "s1"):
+            assert np.array_equal(got[f], want[f])
+        again = srv.submit(10**9, 10**9 + 100)
+        assert srv.wait(again, 600_000).state == "done"
