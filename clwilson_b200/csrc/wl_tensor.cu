@@ -607,9 +607,8 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
     return ok != 0;
 }
 // Waits for the phase, for about limit_ns at most (a step of a wait is bounded
-// by the hardware); false when the limit was reached, with a limit of 0 at once.
+// by the hardware); false when the limit was reached.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint64_t limit_ns) {
-    if (limit_ns == 0) return false;
     if (mbar_try(bar, parity)) return true;
     uint64_t t0, t;
     asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
@@ -778,7 +777,7 @@ k_tensor_gemm(const TensorDesc* __restrict__ desc, const TensorSec* __restrict__
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     uint32_t tmem;
     asm volatile("ld.shared.b32 %0, [%1];" : "=r"(tmem) : "r"(sTmem));
-    bool ok = true;
+    bool ok = wait_ns != 0;       // with a limit of 0 no wait is waited for
 
     if (wid == TG_EPI_WARPS) {
         if (lane == 0) {
@@ -788,7 +787,7 @@ k_tensor_gemm(const TensorDesc* __restrict__ desc, const TensorSec* __restrict__
             const uint8_t* src = w + (uint64_t)(sec.mt0 + it.cb0 * tn) * TN_KB * TG_A_BYTES;
             const uint32_t nblk = ntiles * TN_KB;
             uint32_t s = 0, ph = 0, issued = 0;
-            for (; issued < nblk; ++issued) {
+            for (; ok && issued < nblk; ++issued) {
                 ok = mbar_wait(bEmpty + 8 * s, ph ^ 1, wait_ns);
                 if (!ok) break;
                 mbar_expect(bFull + 8 * s, TG_A_BYTES);
@@ -802,7 +801,7 @@ k_tensor_gemm(const TensorDesc* __restrict__ desc, const TensorSec* __restrict__
         }
     } else if (wid == TG_EPI_WARPS + 1) {
         if (lane == 0) {
-            ok = mbar_wait(bConst, 0, wait_ns);
+            ok = ok && mbar_wait(bConst, 0, wait_ns);
             uint32_t s = 0, ph = 0;
             bool issued = false;
             for (uint32_t t = 0; t < ntiles && ok; ++t) {
